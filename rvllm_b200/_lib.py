@@ -128,6 +128,24 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The CPython module of the launch entry points (``csrc/py_launch.cpp``): the library's functions without the cost
+    of a ctypes call.  Missing is a hard error, as for the library itself."""
+    global _native
+    if _native is None:
+        lib()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RvllmError(E_ARTIFACT, "load", f"rvllm_b200/_native.so cannot be loaded ({e}); build it with "
+                                                 "`python -m rvllm_b200.build`") from e
+        _native = module
+    return _native
+
+
 def last_error() -> str:
     return lib().rvllm_b200_last_error().decode()
 
@@ -147,7 +165,18 @@ def ptr(t):
     return t.data_ptr()
 
 
-def current_stream() -> int:
-    import torch
+_raw_stream = None
 
-    return torch.cuda.current_stream().cuda_stream
+
+def current_stream() -> int:
+    """torch's current stream on the current device.  After the first call (which initialises CUDA) the handle is read
+    without building a torch Stream object: this runs once per launch."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+
+        handle = torch.cuda.current_stream().cuda_stream
+        raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        _raw_stream = (lambda: raw(device())) if raw and device else (lambda: torch.cuda.current_stream().cuda_stream)
+        return handle
+    return _raw_stream()

@@ -5,7 +5,19 @@ from __future__ import annotations
 from dataclasses import dataclass
 
 from . import _lib
-from ._lib import BF16, F16, check, lib, ptr
+from ._lib import BF16, F16, check, lib, native
+
+
+_f16 = None
+
+
+def _float16():
+    global _f16
+    if _f16 is None:
+        import torch
+
+        _f16 = torch.float16
+    return _f16
 
 
 @dataclass
@@ -44,20 +56,17 @@ class PagedDecodeFp8Launcher:
     def launch(self, q_fp8, k_cache, v_cache, out, block_tables, context_lens, workspace=None, k_scale_cache=None,
                v_scale_cache=None, q_scale_cache=None, q_descale=None, k_descale=None, v_descale=None,
                stream=None) -> None:
-        import torch
-
         p = self.params
-        p.validate()
-        dt = F16 if out.dtype == torch.float16 else BF16
-        ws_len = workspace.numel() * workspace.element_size() if workspace is not None else 0
-        check(lib().rvllm_paged_decode_fp8(ptr(q_fp8), ptr(k_cache), ptr(v_cache), ptr(out), dt, ptr(block_tables),
-                                           ptr(context_lens), ptr(workspace), ws_len, ptr(k_scale_cache),
-                                           ptr(v_scale_cache), ptr(q_scale_cache), ptr(q_descale), ptr(k_descale),
-                                           ptr(v_descale), p.scale, p.num_seqs, p.num_heads, p.num_kv_heads,
-                                           p.head_dim, p.block_size, p.max_blocks_per_seq, p.num_blocks_total,
-                                           p.window_size_left, _lib.current_stream() if stream is None else stream),
-              "paged_decode_fp8")
-
+        rc = native().rvllm_paged_decode_fp8(q_fp8, k_cache, v_cache, out, F16 if out.dtype == _float16() else BF16,
+                                             block_tables, context_lens, workspace,
+                                             0 if workspace is None else workspace.nbytes, k_scale_cache, v_scale_cache,
+                                             q_scale_cache, q_descale, k_descale, v_descale, p.scale, p.num_seqs,
+                                             p.num_heads, p.num_kv_heads, p.head_dim, p.block_size,
+                                             p.max_blocks_per_seq, p.num_blocks_total, p.window_size_left,
+                                             _lib.current_stream() if stream is None else stream)
+        if rc:
+            p.validate()  # (the same checks the call has just made: names the parameter set that failed)
+            check(rc, "paged_decode_fp8")
 
     def quant_workspace_bytes(self) -> int:
         p = self.params
@@ -68,12 +77,12 @@ class PagedDecodeFp8Launcher:
                      k_descale=None, v_descale=None, stream=None) -> None:
         """Attention + LSE combine + per-token FP8 quantisation of the [heads*head_dim] row in one call."""
         p = self.params
-        p.validate()
-        check(lib().rvllm_paged_decode_fp8_quant(ptr(q_fp8), ptr(k_cache), ptr(v_cache), ptr(out_fp8), ptr(out_scale),
-                                                 round_dtype, ptr(block_tables), ptr(context_lens), ptr(workspace),
-                                                 workspace.numel() * workspace.element_size(), ptr(k_scale_cache),
-                                                 ptr(v_scale_cache), ptr(q_scale_cache), ptr(q_descale), ptr(k_descale),
-                                                 ptr(v_descale), p.scale, p.num_seqs, p.num_heads, p.num_kv_heads,
-                                                 p.head_dim, p.block_size, p.max_blocks_per_seq, p.num_blocks_total,
-                                                 p.window_size_left, _lib.current_stream() if stream is None else stream),
-              "paged_decode_fp8_quant")
+        rc = native().rvllm_paged_decode_fp8_quant(q_fp8, k_cache, v_cache, out_fp8, out_scale, round_dtype, block_tables,
+                                                   context_lens, workspace, workspace.nbytes, k_scale_cache, v_scale_cache,
+                                                   q_scale_cache, q_descale, k_descale, v_descale, p.scale, p.num_seqs,
+                                                   p.num_heads, p.num_kv_heads, p.head_dim, p.block_size,
+                                                   p.max_blocks_per_seq, p.num_blocks_total, p.window_size_left,
+                                                   _lib.current_stream() if stream is None else stream)
+        if rc:
+            p.validate()
+            check(rc, "paged_decode_fp8_quant")

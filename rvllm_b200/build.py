@@ -1,6 +1,7 @@
 """Builds the sm_100a artifacts of the package, in-tree:
 
   rvllm_b200/librvllm_b200.so        the C-ABI shared library (all kernels + host launchers)
+  rvllm_b200/_native.so              CPython module over that library's launch entry points
   rvllm_b200/kernels/sm_100/*.ptx    PTX modules carrying the reference's entry-point names
   rvllm_b200/kernels/sm_100/manifest.json (+ manifest.sha256)
 
@@ -16,10 +17,12 @@ import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "librvllm_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")
 KDIR = os.path.join(HERE, "kernels", "sm_100")
 OBJ = os.path.join(HERE, "build")
 
@@ -117,6 +120,15 @@ def build_library(force=False, verbose=False):
     return LIB
 
 
+def build_native(force=False):
+    """The CPython module of the launch entry points, linked against the library beside it."""
+    src = os.path.join(CSRC, "py_launch.cpp")
+    if force or _newer(NATIVE, [src, os.path.join(os.path.dirname(HERE), "include", "rvllm_b200.h"), LIB]):
+        _run(["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], src, "-o", NATIVE,
+              "-L", HERE, "-l:librvllm_b200.so", "-Wl,-rpath,$ORIGIN"])
+    return NATIVE
+
+
 def _sha256(path):
     h = hashlib.sha256()
     with open(path, "rb") as f:
@@ -159,6 +171,7 @@ def build_ptx(force=False):
 
 def build_all(force=False, verbose=False):
     build_library(force=force, verbose=verbose)
+    build_native(force=force)
     build_ptx(force=force)
     return LIB
 

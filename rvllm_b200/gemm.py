@@ -4,15 +4,19 @@ the C ABI; these wrappers only marshal torch tensors.  IMPL_* selects the kernel
 from __future__ import annotations
 
 from . import _lib
-from ._lib import OUT_BF16, OUT_F16, OUT_F32, check, lib, ptr
+from ._lib import OUT_BF16, OUT_F16, OUT_F32, check, lib, native
 
 IMPL_AUTO, IMPL_STREAM, IMPL_TCGEN05 = 0, 1, 2
 
+_OUT_KINDS = {}  # torch dtype -> RVLLM_OUT_*, filled on first use (importing the package does not import torch)
+
 
 def _out_kind(t) -> int:
-    import torch
+    if not _OUT_KINDS:
+        import torch
 
-    return {torch.float16: OUT_F16, torch.bfloat16: OUT_BF16, torch.float32: OUT_F32}[t.dtype]
+        _OUT_KINDS.update({torch.float16: OUT_F16, torch.bfloat16: OUT_BF16, torch.float32: OUT_F32})
+    return _OUT_KINDS[t.dtype]
 
 
 def fp8_gemm_channelscale(out, a_fp8, w_fp8, a_scale, w_scale, residual=None, impl=IMPL_AUTO, workspace=None,
@@ -20,10 +24,11 @@ def fp8_gemm_channelscale(out, a_fp8, w_fp8, a_scale, w_scale, residual=None, im
     """out[M, N] = cast(a_scale[m] * (w_scale[n] * A[M, K] . W[N, K]^T) (+ residual))."""
     M, K = a_fp8.shape
     N = w_fp8.shape[0]
-    ws_ptr, ws_len = (ptr(workspace), workspace.numel() * workspace.element_size()) if workspace is not None else (None, 0)
-    check(lib().rvllm_fp8_gemm_channelscale(ptr(out), _out_kind(out), ptr(a_fp8), ptr(w_fp8), ptr(a_scale),
-                                            ptr(w_scale), ptr(residual), M, N, K, impl, ws_ptr, ws_len,
-                                            _lib.current_stream() if stream is None else stream), "fp8_gemm_channelscale")
+    rc = native().rvllm_fp8_gemm_channelscale(out, _out_kind(out), a_fp8, w_fp8, a_scale, w_scale, residual, M, N, K, impl,
+                                              workspace, 0 if workspace is None else workspace.nbytes,
+                                              _lib.current_stream() if stream is None else stream)
+    if rc:
+        check(rc, "fp8_gemm_channelscale")
 
 
 def gateup_workspace_bytes(M: int, I: int, K: int) -> int:
@@ -34,11 +39,11 @@ def fp8_gemm_gateup_act_quant(out_fp8, out_scale, a_fp8, w_fp8, a_scale, w_scale
                               impl=IMPL_AUTO, stream=None) -> None:
     M, K = a_fp8.shape
     I = w_fp8.shape[0] // 2
-    check(lib().rvllm_fp8_gemm_gateup_act_quant(ptr(out_fp8), ptr(out_scale), ptr(a_fp8), ptr(w_fp8), ptr(a_scale),
-                                                ptr(w_scale), M, I, K, act, dtype, impl, ptr(workspace),
-                                                workspace.numel() * workspace.element_size(),
-                                                _lib.current_stream() if stream is None else stream),
-          "fp8_gemm_gateup_act_quant")
+    rc = native().rvllm_fp8_gemm_gateup_act_quant(out_fp8, out_scale, a_fp8, w_fp8, a_scale, w_scale, M, I, K, act, dtype, impl,
+                                                  workspace, workspace.nbytes,
+                                                  _lib.current_stream() if stream is None else stream)
+    if rc:
+        check(rc, "fp8_gemm_gateup_act_quant")
 
 
 def tc_status(reset: bool = True) -> int:
