@@ -317,11 +317,12 @@ int rvllm_fp8_gemm_gateup_act_quant(void* out_fp8, float* out_scale, const void*
     const size_t stage = ((size_t)M * 2 * (size_t)I * 2 + 255) & ~(size_t)255;
     if (!workspace || !rv_aligned(workspace, 256) || workspace_size < rvllm_fp8_gemm_gateup_workspace(M, I, K))
         return rv_fail(RVLLM_E_WORKSPACE, "gate-up workspace missing, misaligned or too small");
-    // One launch where the layer-block kernel's gate|up stage takes the shape (batch <= 32, K a multiple of 128 up to
-    // 6144, I a multiple of 64 up to 4 * K): gate and up rows of the same 64 columns are one 128-row operand, the
-    // epilogue rounds both to the 16-bit type, multiplies, keeps the products on chip, the grid meets once for the
-    // row maxima and quantises — the [M, 2*I] intermediate never reaches HBM.  Same bytes as the two launches below.
-    if (impl == 0 || impl == 3) {
+    // The choice left to the library (impl 0) is the two launches below.  The single launch (impl 3: the layer-block
+    // kernel's gate|up stage, whose [M, 2*I] intermediate never reaches HBM) loses to them at every size it takes: its
+    // grid barrier and the barrier-word memset in front cost more than the intermediate's round trip through L2, and it
+    // cannot start under programmatic dependent launch.  Measured, us per call, single / two launches: [2*2048 x 512]
+    // 23 / 8, [2*3456 x 1152] 26 / 10, [2*14336 x 4096] 48 / 32-38, [2*21504 x 5376] 64 / 42-45, M = 1 to 32.
+    if (impl == 3) {
         const bool takes = rvblk::blk_shape_ok(M, K, I, K) && rv_aligned(a_fp8, 16) && rv_aligned(w_fp8, 16) &&
                            rv_aligned(out_fp8, 16) && a_scale && w_scale && out_scale &&
                            workspace_size >= 256 + rvblk::blk_amax_bytes(I);
@@ -356,13 +357,13 @@ int rvllm_fp8_gemm_gateup_act_quant(void* out_fp8, float* out_scale, const void*
             if (rc == 0) return RVLLM_OK;
             if (rc != -3) return rc;
         }
-        if (impl == 3) return rv_fail(RVLLM_E_UNSUPPORTED, "gate-up single launch: shape not taken");
+        return rv_fail(RVLLM_E_UNSUPPORTED, "gate-up single launch: shape not taken");
     }
     // Two launches.  The projection lands in the 16-bit type the standalone chain would use, so the
     // activation + re-quantisation sees bit-identical inputs either way.
     GemmArgs g = {workspace, dtype == RVLLM_F16 ? RVLLM_OUT_F16 : RVLLM_OUT_BF16, a_fp8, w_fp8, a_scale, w_scale,
                   nullptr, M, 2 * I, K};
-    rc = run_gemm(g, impl == 3 ? 0 : impl, (char*)workspace + stage, workspace_size - stage, (cudaStream_t)stream);
+    rc = run_gemm(g, impl, (char*)workspace + stage, workspace_size - stage, (cudaStream_t)stream);
     if (rc) return rc;
     return rvllm_fused_act_mul_fp8_quant_launch((uint32_t)M, (uint32_t)I, act, out_fp8, out_scale, workspace, dtype,
                                                 stream);
