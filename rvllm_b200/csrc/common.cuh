@@ -138,4 +138,16 @@ __device__ __forceinline__ uint4 ld_stream128(const void* p) {
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// One lane of a converged warp.  The producer's and the issuer's loops run on all lanes with one elected lane doing the
+// work: under a branch on the lane number the compiler cannot keep descriptors and addresses in uniform registers, and
+// moving them there for every instruction made the issuing thread slower than the tensor pipe (about 80 cycles per MMA
+// and 450 per K block on top).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// (the warp's number through a shuffle, so that the compiler knows it is the same in all lanes)
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
 }  // namespace rv

@@ -286,7 +286,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     cg::cluster_group cluster = cg::this_cluster();
     const int S = gridDim.y, split = blockIdx.y;
     const int n0 = blockIdx.x * TILE_W, m0 = blockIdx.z * BN;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = rv::uniform_warp(), lane = threadIdx.x & 31;
     const int kb_lo = (int)((long long)split * p.kblocks / S);
     const int kb_hi = (int)((long long)(split + 1) * p.kblocks / S);
     const int nkb = kb_hi - kb_lo;
@@ -368,49 +368,54 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     if (push && (!push_ring || push_mbar)) cluster_arrive();
 
     if (warp == 0) {
-        if (lane == 0) {
-            const int pre = nkb < STAGES ? nkb : STAGES;  // (their weight tiles are already on the way)
-            if (!A16) {
-                rv::pdl_wait();
-                trace_point(p.trace, 1);  // the kernel ahead in the stream is complete
-                for (int i = 0; i < pre; i++)
-                    tma_load_2d(ring + (size_t)i * C::STAGE_BYTES + TILE_W * BK, &map_a, (kb_lo + i) * BK, m0, full + i);
-            }
-            bool alive = true;
-            for (int i = pre; i < nkb; i++) {
-                const int s = i % STAGES;
-                const uint32_t ph = (uint32_t)(i / STAGES) & 1u;
-                alive = mbar_wait(empty + s, ph ^ 1u, 1);
-                if (!alive) break;
-                uint8_t* w_dst = ring + (size_t)s * C::STAGE_BYTES;
+        const int pre = nkb < STAGES ? nkb : STAGES;  // (their weight tiles are already on the way)
+        const bool one = rv::elect_one();
+        if (!A16) {
+            rv::pdl_wait();
+            if (lane == 0) trace_point(p.trace, 1);  // the kernel ahead in the stream is complete
+            for (int i = 0; i < pre; i++)
+                if (one) tma_load_2d(ring + (size_t)i * C::STAGE_BYTES + TILE_W * BK, &map_a, (kb_lo + i) * BK, m0, full + i);
+        }
+        int s = 0;
+        uint32_t ph = 0;
+        for (int i = pre; i < nkb; i++) {
+            if (!mbar_wait(empty + s, ph, 1)) break;
+            uint8_t* w_dst = ring + (size_t)s * C::STAGE_BYTES;
+            if (one) {
                 mbar_expect_tx(full + s, A16 ? TILE_W * BK : C::STAGE_BYTES);
                 tma_load_2d(w_dst, &map_w, (kb_lo + i) * BK, n0, full + s);
                 if (!A16) tma_load_2d(w_dst + TILE_W * BK, &map_a, (kb_lo + i) * BK, m0, full + s);
             }
+            if (++s == STAGES) {
+                s = 0;
+                ph ^= 1u;
+            }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(BN);
-            bool alive = true;
-            for (int i = 0; i < nkb && alive; i++) {
-                const int s = i % STAGES;
-                const uint32_t ph = (uint32_t)(i / STAGES) & 1u;
-                alive = mbar_wait(full + s, ph, 2);
-                if (!alive) break;
-                if (i == 0) trace_point(p.trace, 2);  // both operands of the first K block are in shared memory
-                tc_fence_after();
-                const uint32_t w_addr = smem_u32(ring + (size_t)s * C::STAGE_BYTES);
-                const uint64_t adesc = smem_desc_sw128(w_addr);
-                const uint64_t bdesc = smem_desc_sw128(w_addr + TILE_W * BK);
+        constexpr uint32_t idesc = instr_desc(BN);
+        const bool one = rv::elect_one();
+        const uint64_t desc0 = smem_desc_sw128(smem_u32(ring));
+        int s = 0;
+        uint32_t ph = 0;
+        for (int i = 0; i < nkb; i++) {
+            if (!mbar_wait(full + s, ph, 2)) break;
+            if (lane == 0 && i == 0) trace_point(p.trace, 2);  // both operands of the first K block are in shared memory
+            tc_fence_after();
+            const uint64_t adesc = desc0 + (uint64_t)(C::STAGE_BYTES >> 4) * (uint64_t)s, bdesc = adesc + (uint64_t)(TILE_W * BK >> 4);
+            if (one) {
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; k++)
                     umma_f8(tmem_base, adesc + (uint64_t)(k * UMMA_K >> 4), bdesc + (uint64_t)(k * UMMA_K >> 4), idesc,
                             (i > 0 || k > 0) ? 1u : 0u);
                 umma_commit(empty + s);  // frees the stage once these MMAs have read it
             }
-            umma_commit(acc_ready);  // arrives when every MMA issued above has completed
-            trace_point(p.trace, 3);  // the last MMA is issued
+            if (++s == STAGES) {
+                s = 0;
+                ph ^= 1u;
+            }
         }
+        if (one) umma_commit(acc_ready);  // arrives when every MMA issued above has completed
+        if (lane == 0) trace_point(p.trace, 3);  // the last MMA is issued
     }
     if (A16 && warp >= EPI_WARP0) {
         // The four epilogue warps are idle during the main loop: they turn the 16-bit activations into the

@@ -229,7 +229,7 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
 
     rv::pdl_launch();
     const int kvh = blockIdx.x, chunk = blockIdx.y, b = blockIdx.z;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = rv::uniform_warp(), lane = tid & 31;
     const int group = p.heads / p.kv_heads;
     OutT* out = reinterpret_cast<OutT*>(p.out);
 
@@ -365,7 +365,8 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && ntiles > 0) {
+        if (ntiles > 0) {
+            const bool one = rv::elect_one();
             constexpr uint32_t idesc_qk = instr_desc(NQ, false), idesc_pv = instr_desc(NP, true);
             const uint64_t qdesc = desc_kmajor(smem_u32(q_tile)), pdesc = desc_kmajor(smem_u32(p_tile));
             // Issue whichever product has its inputs first: the score MMA of the next tile (its K panels
@@ -398,7 +399,7 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 bool did = false;
                 if (next_qk < ntiles && next_qk <= next_pv + 2) {  // the score tile in TMEM is double buffered
                     const int i = next_qk;
-                    bool ok = i < 2 || mbar_try_wait(s_free + (i & 1), (uint32_t)((i >> 1) - 1) & 1u);
+                    bool ok = one && (i < 2 || mbar_try_wait(s_free + (i & 1), (uint32_t)((i >> 1) - 1) & 1u));
                     int slot[HALVES];
 #pragma unroll
                     for (int h = 0; h < HALVES; h++) {
@@ -410,19 +411,21 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                         slot[h] = sl;
                         ok = ok && prev_consumed(i * UPT + h) && mbar_try_wait(full + sl, (uint32_t)us & 1u);
                     }
-                    if (ok) {
+                    if (__any_sync(0xffffffffu, ok)) {
                         tc_fence_after();
+                        if (one) {
 #pragma unroll
-                        for (int h = 0; h < HALVES; h++) {
-                            const uint64_t kdesc = desc_kmajor(smem_u32(ring + (size_t)slot[h] * UNIT));
-                            const uint64_t qd = qdesc + (uint64_t)((h * NQ * PANEL) >> 4);
+                            for (int h = 0; h < HALVES; h++) {
+                                const uint64_t kdesc = desc_kmajor(smem_u32(ring + (size_t)slot[h] * UNIT));
+                                const uint64_t qd = qdesc + (uint64_t)((h * NQ * PANEL) >> 4);
 #pragma unroll
-                            for (int k = 0; k < PANEL / 32; k++)
-                                umma_f8(tmem_base + (uint32_t)(i & 1) * NQ, kdesc + (uint64_t)(2 * k), qd + (uint64_t)(2 * k),
-                                        idesc_qk, (h > 0 || k > 0) ? 1u : 0u);
-                            umma_commit(empty + slot[h]);
+                                for (int k = 0; k < PANEL / 32; k++)
+                                    umma_f8(tmem_base + (uint32_t)(i & 1) * NQ, kdesc + (uint64_t)(2 * k), qd + (uint64_t)(2 * k),
+                                            idesc_qk, (h > 0 || k > 0) ? 1u : 0u);
+                                umma_commit(empty + slot[h]);
+                            }
+                            umma_commit(s_ready + (i & 1));
                         }
-                        umma_commit(s_ready + (i & 1));
                         next_qk++;
                         advance(q_slot, q_use);
                         did = true;
@@ -430,7 +433,7 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 }
                 if (next_pv < next_qk) {
                     const int i = next_pv;
-                    bool ok = mbar_try_wait(p_ready, (uint32_t)i & 1u);
+                    bool ok = one && mbar_try_wait(p_ready, (uint32_t)i & 1u);
                     int slot[HALVES];
 #pragma unroll
                     for (int h = 0; h < HALVES; h++) {
@@ -442,18 +445,20 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                         slot[h] = sl;
                         ok = ok && prev_consumed(i * UPT + HALVES + h) && mbar_try_wait(full + sl, (uint32_t)us & 1u);
                     }
-                    if (ok) {
+                    if (__any_sync(0xffffffffu, ok)) {
                         tc_fence_after();
+                        if (one) {
 #pragma unroll
-                        for (int h = 0; h < HALVES; h++) {
-                            const uint64_t vdesc = desc_mnmajor(smem_u32(ring + (size_t)slot[h] * UNIT));
+                            for (int h = 0; h < HALVES; h++) {
+                                const uint64_t vdesc = desc_mnmajor(smem_u32(ring + (size_t)slot[h] * UNIT));
 #pragma unroll
-                            for (int k = 0; k < TOK / 32; k++)  // 32 tokens (rows of 128 B) per MMA
-                                umma_f8(tmem_base + C::O_COL + (uint32_t)h * NP, vdesc + (uint64_t)((32 * PANEL * k) >> 4),
-                                        pdesc + (uint64_t)(2 * k), idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
-                            umma_commit(empty + slot[h]);
+                                for (int k = 0; k < TOK / 32; k++)  // 32 tokens (rows of 128 B) per MMA
+                                    umma_f8(tmem_base + C::O_COL + (uint32_t)h * NP, vdesc + (uint64_t)((32 * PANEL * k) >> 4),
+                                            pdesc + (uint64_t)(2 * k), idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
+                                umma_commit(empty + slot[h]);
+                            }
+                            umma_commit(pv_done);
                         }
-                        umma_commit(pv_done);
                         next_pv++;
                         advance(v_slot, v_use);
                         did = true;
@@ -462,7 +467,7 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 if (did) {
                     idle = 0;
                 } else if (++idle > WAIT_LIMIT) {
-                    atomicCAS(&g_status, 0, (2 << 16) | (int)(blockIdx.x & 0xffff));
+                    if (one) atomicCAS(&g_status, 0, (2 << 16) | (int)(blockIdx.x & 0xffff));
                     alive = false;
                 }
             }
