@@ -24,12 +24,12 @@ void rvllm_b200_set_pdl(int enabled);
 int rvllm_b200_get_pdl(void);
 
 /* Overrides of the tcgen05 kernel's automatic choices, for tuning runs: TMA ring depth
- * (2..8) and split-K factor (1..8); 0 restores the automatic choice.  Process-wide. */
+ * (2..8) and split-K factor (1..8); 0 restores the automatic choice.  Process-wide.  They and the two hooks below
+ * concern launches of up to 32 rows: the CTA-pair kernel that takes larger ones has its own plan. */
 void rvllm_fp8_gemm_tc_tune(int stages, int splits);
-/* Form of the split-K reduction inside a cluster: 0 automatic (batch tiles up to 32 rows: partials are pushed into
- * the finishing CTA's receive buffer and every sender arrives on the owner's mbarrier; 64- and 128-row tiles: pushed
- * into the peers' idle rings between two cluster barriers; 256-row tiles: pulled out of the peers' rings), 1 always
- * pull, 2 the same as 0, 3 the small-tile push completed by one cluster barrier instead of the mbarrier arrivals
+/* Form of the split-K reduction inside a cluster: 0 automatic (partials are pushed into the finishing CTA's receive
+ * buffer and every sender arrives on the owner's mbarrier), 1 always pull out of the peers' rings, 2 the same as 0,
+ * 3 the push completed by one cluster barrier instead of the mbarrier arrivals
  * (1.3 us per layer slower in the decode graph; kept as a cross-check).  All forms sum in cluster-rank order, so their
  * results are bitwise equal (tested). */
 void rvllm_fp8_gemm_tc_reduce(int mode);
@@ -45,7 +45,7 @@ void rvllm_fp8_gemm_tc_split_target(int ctas);
  * The stamps exist only in a library built with RVLLM_TC_TRACE=1 (they cost the decode step 1.2 % even when off);
  * otherwise setting a buffer returns RVLLM_E_UNSUPPORTED. */
 int rvllm_fp8_gemm_tc_trace(void* device_u64_buffer, int slots);
-/* Split-K factor of one weight shape [N, K] (batch tiles up to 128 rows), four slots; splits 0 clears the slot. */
+/* Split-K factor of one weight shape [N, K], four slots; splits 0 clears the slot. */
 void rvllm_fp8_gemm_tc_split_for(int slot, int N, int K, int splits);
 
 /* Overrides for tuning runs (0 restores the default): CTAs the grid aims for, the fewest tokens

@@ -7,6 +7,7 @@
 #include "host_util.h"
 #include "fp8_gemm_stream.cuh"
 #include "fp8_gemm_tc.cuh"
+#include "fp8_gemm_pair.cuh"
 #include "fp8_layer_block.cuh"
 
 extern "C" {
@@ -136,6 +137,7 @@ int run_gemm(const GemmArgs& g, int impl, void* workspace, size_t workspace_size
         t.M = g.M;
         t.N = g.N;
         t.K = g.K;
+        if (rvpair::prefer_pair(g.M, g.N, g.K)) return rvpair::launch_pair(t, s);
         return rvtc::launch(t, workspace, workspace_size, s);
     }
     if (impl != 1) return rv_fail(RVLLM_E_INVALID, "impl must be 0, 1 or 2");
@@ -248,7 +250,12 @@ int rvllm_fp8_gemm_qkv_rope_fp8kv(const void* a_fp8, const void* w_fp8, const fl
     t.K = K;
     rvtc::RopeKv rk = {(uint8_t*)q_fp8, q_scale, (uint8_t*)k_cache, (uint8_t*)v_cache, k_scale_cache, v_scale_cache,
                        cos_table, sin_table, positions, slot_mapping, heads, kv_heads, max_positions, num_cache_slots};
-    const int rc = rvtc::launch_qkv_rope(t, rk, dtype == RVLLM_F16 ? 0 : 1, (cudaStream_t)stream);
+    const int dt = dtype == RVLLM_F16 ? 0 : 1;
+    if (M > 32 && (!rv_aligned(cos_table, 4) || !rv_aligned(sin_table, 4) || !rv_aligned(q_fp8, 2) || !rv_aligned(k_cache, 2) ||
+                   !rv_aligned(v_cache, 2)))
+        return rv_fail(RVLLM_E_UNSUPPORTED, "fused QKV epilogue: tables must be 4-byte, Q and caches 2-byte aligned above 32 rows");
+    const int rc = M > 32 ? rvpair::launch_pair_qkv_rope(t, rk, dt, (cudaStream_t)stream)
+                          : rvtc::launch_qkv_rope(t, rk, dt, (cudaStream_t)stream);
     if (rc == -3) return RVLLM_E_UNSUPPORTED;  // message already recorded
     return rc;
 }
@@ -400,7 +407,8 @@ int rvllm_fp8_gemm_lm_head_argmax(int32_t* out_tokens, const void* a_fp8, const 
     t.arg_val = (float*)workspace;
     t.arg_idx = (int*)((char*)workspace + need / 2);
     t.softcap = softcap;
-    rc = rvtc::launch_argmax(t, out_tokens, (cudaStream_t)stream);
+    rc = M > 32 ? rvpair::launch_pair_argmax(t, (cudaStream_t)stream) : rvtc::launch_argmax(t, (cudaStream_t)stream);
+    if (rc == 0) rc = rvtc::launch_argmax_merge(t, out_tokens, (cudaStream_t)stream);
     if (rc == -3) return RVLLM_E_UNSUPPORTED;
     return rc;
 }

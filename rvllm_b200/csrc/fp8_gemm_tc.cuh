@@ -6,8 +6,8 @@
 //
 // The roles are swapped relative to a textbook GEMM so that decode-sized batches still
 // fill the 128-lane tensor-core tile: a 128-row slab of W is the MMA's M operand, the
-// batch rows are its N operand (16..256), so the accumulator in TMEM is D^T
-// [128 weight rows (lanes) x BN batch rows (columns)] in f32.
+// batch rows are its N operand (16 or 32; larger batches run on CTA pairs, fp8_gemm_pair.cuh),
+// so the accumulator in TMEM is D^T [128 weight rows (lanes) x BN batch rows (columns)] in f32.
 //
 //   warp 0   : TMA producer — one lane issues cp.async.bulk.tensor.2d loads of a
 //              128 x 128 B weight tile and a BN x 128 B activation tile per stage
@@ -280,7 +280,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     uint64_t* acc_ready = empty + MAX_STAGES;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_ready + 1);
     uint64_t* recv_bar = reinterpret_cast<uint64_t*>(header + 512);  // push reduction: all partials for this CTA have landed
-    uint64_t* free_bar = recv_bar + 1;                               // ring push: every CTA of the cluster is done with its ring
     const int STAGES = p.stages;
 
     cg::cluster_group cluster = cg::this_cluster();
@@ -306,7 +305,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         mbar_init(acc_ready, 1);
         mbar_init(recv_bar, (uint32_t)gridDim.y * 4u);  // one arrival per epilogue warp of every CTA of the cluster
-        mbar_init(free_bar, (uint32_t)gridDim.y);       // one arrival per CTA of the cluster
         fence_barrier_init();
         // This thread is also the TMA producer.  Weights never depend on the previous kernel: fill the ring
         // with weight tiles right away (before the block even meets; the barriers are this thread's own),
@@ -360,12 +358,9 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (threadIdx.x == 0) trace_point(p.trace, 1);  // predecessor complete, row scales known
     }
     const bool push = S > 1 && p.push != 0;
-    // push == 3: the receive buffer is the (by then idle) ring itself — batch tiles of 64 / 128 rows, whose partials
-    // would not fit behind it.  The cluster then meets after the main loops instead ("every ring is free").
-    const bool push_ring = BN >= 64 && push && p.push >= 3;  // (a compile-time "no" for the small tiles)
-    const bool push_mbar = p.push == 2 || p.push == 3;       // completion: arrivals on the owners' mbarriers (else a cluster barrier)
+    const bool push_mbar = p.push == 2;  // completion: arrivals on the owners' mbarriers (else a cluster barrier)
     // "this CTA runs": peers wait for it (long since complete) before their first remote store or arrival
-    if (push && (!push_ring || push_mbar)) cluster_arrive();
+    if (push) cluster_arrive();
 
     if (warp == 0) {
         const int pre = nkb < STAGES ? nkb : STAGES;  // (their weight tiles are already on the way)
@@ -467,7 +462,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // own rank), the cluster meets once, and each CTA sums the S slots of its columns in rank order:
         // one barrier, no remote loads, bitwise reproducible.  Measured ~2.5 us per launch less than
         // pulling the partials out of the peers' rings (two barriers and a remote-load round trip).
-        float* recv = reinterpret_cast<float*>(push_ring ? ring : ring + (size_t)STAGES * C::STAGE_BYTES);  // [S][LC][TILE_W]
+        float* recv = reinterpret_cast<float*>(ring + (size_t)STAGES * C::STAGE_BYTES);  // [S][LC][TILE_W]
         const int LC = (BN + S - 1) / S;
         constexpr int PRE = 3;
         float pre_a[PRE], pre_w[PRE], pre_res[PRE];
@@ -513,29 +508,12 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
         bool ready = true;
-        if (push_ring) {
-            // own MMAs complete = every load into this CTA's ring has landed and been read: the ring is free;
-            // once the whole cluster has said so, every ring may be written
-            if (warp >= EPI_WARP0 && nkb > 0) ready = mbar_wait(acc_ready, 0, 3);
-            if (threadIdx.x == EPI_WARP0 * 32) trace_point(p.trace, 4);  // the accumulator is complete
-            if (push_mbar) {
-                // one warp tells every CTA of the cluster (itself included); the pushing warps wait for all of them
-                cluster_wait();  // (every CTA runs: its barriers exist)
-                if (warp == EPI_WARP0) {
-                    __syncwarp();
-                    if (lane < S) mbar_arrive_peer(free_bar, (uint32_t)lane);
-                }
-                if (warp >= EPI_WARP0) mbar_wait_cluster(free_bar, 0, 8);
-            } else {
-                cluster_arrive();
-            }
-        }
-        if (!(push_ring && push_mbar)) cluster_wait();  // every CTA of the cluster is running (and, in the ring + barrier form, done with its ring)
+        cluster_wait();  // every CTA of the cluster is running
         if (warp >= EPI_WARP0) {
             const int quarter = warp & 3;
             const int r = quarter * 32 + lane;
-            if (!push_ring && nkb > 0) ready = mbar_wait(acc_ready, 0, 3);
-            if (!push_ring && threadIdx.x == EPI_WARP0 * 32) trace_point(p.trace, 4);  // the accumulator is complete
+            if (nkb > 0) ready = mbar_wait(acc_ready, 0, 3);
+            if (threadIdx.x == EPI_WARP0 * 32) trace_point(p.trace, 4);  // the accumulator is complete
             tc_fence_after();
             const uint32_t slot = smem_u32(recv) + (uint32_t)((split * LC) * TILE_W + r) * 4u;  // [split][0][r]
             uint32_t owner = 0, lc_off = 0;
@@ -715,24 +693,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
         auto as_col = [&](int c) -> float { return A16 ? s_ascale[c] : s_as[c]; };  // (S == 1 only)
-        // residual values one 16-column group ahead (out and residual may be one buffer: every element is read
-        // before any store of its group, and by the thread that stores it)
-        // (256-row batch tiles only, which run one CTA per SM: the smaller ones count on three, and the registers
-        // this costs would take the third away)
-        constexpr bool RES_AHEAD = RES && BN >= 256;
-        float res_nx[RES_AHEAD ? 16 : 1];
-        auto fetch_res = [&](int c0) {
-            if constexpr (RES_AHEAD) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int m = m0 + c0 + j;
-                    res_nx[j] = (S == 1 && c0 + j < BN && m < p.M && n < p.N)
-                                    ? rv::T16<OutT>::to_f32(reinterpret_cast<const OutT*>(p.residual)[(size_t)m * p.N + n])
-                                    : 0.0f;
-                }
-            }
-        };
-        fetch_res(0);
         bool ready = true;
         if (nkb > 0) ready = mbar_wait(acc_ready, 0, 3);
         if (threadIdx.x == EPI_WARP0 * 32) trace_point(p.trace, 4);  // the accumulator is complete
@@ -746,12 +706,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             } else {
 #pragma unroll
                 for (int j = 0; j < 16; j++) v[j] = 0u;
-            }
-            float res_cur[RES_AHEAD ? 16 : 1];
-            if constexpr (RES_AHEAD) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) res_cur[j] = res_nx[j];
-                if (S == 1) fetch_res(c0 + 16);
             }
             if constexpr (ARG) {
                 // the logit this element would have been (soft-capped), into the idle ring as [batch row][channel]
@@ -777,8 +731,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         } else {
                             if (RES)
                                 val = fmaf(as_col(c0 + j), ws * __uint_as_float(v[j]),
-                                           RES_AHEAD ? res_cur[RES_AHEAD ? j : 0]
-                                                     : rv::T16<OutT>::to_f32(reinterpret_cast<const OutT*>(p.residual)[o]));
+                                           rv::T16<OutT>::to_f32(reinterpret_cast<const OutT*>(p.residual)[o]));
                             reinterpret_cast<OutT*>(p.out)[o] = rv::T16<OutT>::from_f32_sat(val);
                         }
                     }
@@ -1080,12 +1033,8 @@ int launch_one(const TcArgs& g, int splits, int stages, cudaStream_t s, const Ro
     auto kern = fp8_gemm_tc_kernel<BN, EPI, OutT>;
     // Split-K with a small batch tile: push reduction (needs its receive buffer behind the ring);
     // otherwise the partial tile is parked in the ring itself, which must be large enough for it.
-    const bool push = splits > 1 && BN <= 32 && tune().reduce != 1;
-    // 64- and 128-row batch tiles: push as well, into the peers' idle rings (the partials would not fit behind them)
-    const bool push_ring = splits > 1 && (BN == 64 || BN == 128) && tune().reduce != 1 &&
-                           (EPI == EPI_SCALE || EPI == EPI_RESIDUAL || EPI == EPI_F32 || EPI == EPI_QKV_ROPE);
-    const int ring_recv_bytes = push_ring ? splits * ((BN + splits - 1) / splits) * TILE_W * 4 : 0;
-    const int min_stages = (push || push_ring) ? 2 : C::MIN_STAGES;
+    const bool push = splits > 1 && tune().reduce != 1;
+    const int min_stages = push ? 2 : C::MIN_STAGES;
     if (stages < min_stages) stages = min_stages;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
     // dynamic shared memory this instantiation may ask for: the 227 KB per-CTA limit less its static arrays
@@ -1095,9 +1044,8 @@ int launch_one(const TcArgs& g, int splits, int stages, cudaStream_t s, const Ro
     static RvDeviceOnce smem_once;  // per kernel instantiation and device: allow the largest ring once
     {
         int most = MAX_STAGES;
-        const bool may_push = BN <= 32;  // the largest footprint this instantiation can be launched with
-        while (most > C::MIN_STAGES && C::smem_bytes(most, may_push) > SMEM_LIMIT) most--;
-        if (rv_allow_smem(smem_once, kern, C::smem_bytes(most, may_push)))
+        while (most > C::MIN_STAGES && C::smem_bytes(most, true) > SMEM_LIMIT) most--;
+        if (rv_allow_smem(smem_once, kern, C::smem_bytes(most, true)))
             return rvhost::fail_msg(-2, "cannot raise dynamic shared memory for the tcgen05 GEMM");
     }
     TcParams p;
@@ -1112,8 +1060,7 @@ int launch_one(const TcArgs& g, int splits, int stages, cudaStream_t s, const Ro
     p.stages = stages;
     // completion of the push: arrivals on the owners' mbarriers (2, the default: measured 1.3 us per layer faster in
     // the decode graph than the cluster-wide barrier) or one cluster barrier (1, tuning value 3)
-    // (values: 1 small tiles + cluster barrier, 2 small tiles + mbarriers, 3 ring + mbarriers, 4 ring + cluster barrier)
-    p.push = push ? (tune().reduce == 3 ? 1 : 2) : push_ring ? (tune().reduce == 3 ? 4 : 3) : 0;
+    p.push = push ? (tune().reduce == 3 ? 1 : 2) : 0;
     p.rope = rope ? *rope : RopeKv{};
     p.a16 = g.a16;
     p.amax_part = g.amax_part;
@@ -1128,16 +1075,14 @@ int launch_one(const TcArgs& g, int splits, int stages, cudaStream_t s, const Ro
     }
     if (EPI == EPI_ARGMAX && (splits != 1 || !g.arg_val || !g.arg_idx))
         return rvhost::fail_msg(-3, "the argmax epilogue needs an unsplit launch and its partial buffers");
-    if (EPI == EPI_RESIDUAL_A16 && (!g.a16 || !g.amax_part || g.amax_parts <= 0 || BN > 32))
-        return rvhost::fail_msg(-3, "the 16-bit activation form needs a16, partial maxima and a batch tile of at most 32 rows");
-    if (EPI == EPI_QKV_ROPE && (!(push || push_ring) || !rope))
-        return rvhost::fail_msg(-3, "the fused QKV epilogue needs a split-K launch with a batch tile of at most 128 rows");
+    if (EPI == EPI_RESIDUAL_A16 && (!g.a16 || !g.amax_part || g.amax_parts <= 0 ))
+        return rvhost::fail_msg(-3, "the 16-bit activation form needs a16 and partial maxima");
+    if (EPI == EPI_QKV_ROPE && (!push || !rope))
+        return rvhost::fail_msg(-3, "the fused QKV epilogue needs a split-K launch in the push form");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((g.N + TILE_W - 1) / TILE_W, splits, (g.M + BN - 1) / BN);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = C::smem_bytes(stages, push);
-    if (push_ring && stages * C::STAGE_BYTES < ring_recv_bytes)  // a few columns more than the ring holds (S not a power of two)
-        cfg.dynamicSmemBytes += ring_recv_bytes - stages * C::STAGE_BYTES;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1173,18 +1118,9 @@ int launch_epi(const TcArgs& g, int splits, int stages, cudaStream_t s) {
 inline int pick_splits(int M, int N, int K, int bn) {
     const int tiles = ((N + TILE_W - 1) / TILE_W) * ((M + bn - 1) / bn);
     const int kblocks = (K + BK - 1) / BK;
-    // 256-row batch tiles (M > 128) are tensor-bound, one CTA per SM: split only while the tiles leave SMs idle
-    // (measured at M = 512 on the QKV shape: 117 us split three ways with the pull reduction, against 155 us for
-    // four times the work unsplit)
-    if (bn >= 256) {
-        int s2 = 148 / tiles;
-        if (s2 > 8) s2 = 8;
-        while (s2 > 1 && kblocks / s2 < 4) s2--;
-        return s2 < 1 ? 1 : s2;
-    }
     for (int i = 0; i < 4; i++) {
         const long long e = tune().split_for[i].load();
-        if (e != 0 && (e >> 40) == N && ((e >> 8) & 0xffffffffll) == K && bn <= 128) return (int)(e & 0xff);
+        if (e != 0 && (e >> 40) == N && ((e >> 8) & 0xffffffffll) == K) return (int)(e & 0xff);
     }
     const int target = tune().split_target.load() > 0 ? tune().split_target.load() : 360;
     int s = (target + tiles / 2) / tiles;
@@ -1196,14 +1132,12 @@ inline int pick_splits(int M, int N, int K, int bn) {
 
 // Ring depth: a shallow ring lets three CTAs share an SM, so one CTA's prologue / epilogue overlaps
 // the others' streaming; measured faster than a deeper ring with fewer CTAs per SM on every decode
-// shape (gate|up at M = 32: 93 % vs 58 % of the HBM peak with 3 vs 8 stages; at M = 128: 77 % vs
-// 56 % with 2 vs 3 stages).  ~60-66 KB per CTA either way: 3 stages of 20-24 KB up to a 64-row batch
-// tile, 2 stages of 32 KB for a 128-row one.
+// shape (gate|up at M = 32: 93 % vs 58 % of the HBM peak with 3 vs 8 stages).  ~60-66 KB per CTA: 3 stages of 18-20 KB.
 inline int pick_stages(int bn, int splits) {
     // split launches with the push reduction: the ring shares the CTA's ~66 KB with the receive buffer (20 KB for a
     // 32-row batch tile: two stages; 12 KB for a 16-row one: three stages, measured 5 % faster on the batch-1 step)
-    if (bn <= 32 && splits > 1) return bn <= 16 ? 3 : 2;
-    return bn <= 64 ? 3 : bn == 128 ? 2 : 4;
+    if (splits > 1) return bn <= 16 ? 3 : 2;
+    return 3;
 }
 
 // The launch plan of a shape: batch tile, split-K factor, ring depth.
@@ -1212,7 +1146,7 @@ struct Plan {
 };
 inline Plan plan_for(int M, int N, int K) {
     Plan pl;
-    pl.bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+    pl.bn = M <= 16 ? 16 : 32;
     const int t_splits = tune().splits.load(), t_stages = tune().stages.load();
     pl.splits = t_splits > 0 ? t_splits : pick_splits(M, N, K, pl.bn);
     pl.kblocks = (K + BK - 1) / BK;
@@ -1226,37 +1160,22 @@ inline int launch(const TcArgs& g, void*, size_t, cudaStream_t s) {
     if (g.K % 16 != 0) return rvhost::fail_msg(-3, "tcgen05 GEMM needs K to be a multiple of 16");
     const Plan pl = plan_for(g.M, g.N, g.K);
     const int bn = pl.bn, splits = pl.splits, stages = pl.stages;
-    switch (bn) {
-        case 16: return launch_epi<16>(g, splits, stages, s);
-        case 32: return launch_epi<32>(g, splits, stages, s);
-        case 64: return launch_epi<64>(g, splits, stages, s);
-        case 128: return launch_epi<128>(g, splits, stages, s);
-        default: return launch_epi<256>(g, splits, stages, s);
-    }
+    return bn == 16 ? launch_epi<16>(g, splits, stages, s) : launch_epi<32>(g, splits, stages, s);
 }
 
 // QKV projection with RoPE, Q quantisation and the paged FP8 KV write in the epilogue.  head_dim is 128
 // (one weight tile per head), N = (heads + 2 * kv_heads) * 128, M <= 32.  dtype: 0 f16, 1 bf16 (the type
 // the unfused GEMM would have stored, and of the cos / sin tables).  -3: shape not taken, use the two kernels.
 inline int launch_qkv_rope(const TcArgs& g, const RopeKv& rk, int dtype, cudaStream_t s) {
-    if (g.K % 16 != 0 || g.M > 128 || g.N != (rk.heads + 2 * rk.kv_heads) * TILE_W)
+    if (g.K % 16 != 0 || g.M > 32 || g.N != (rk.heads + 2 * rk.kv_heads) * TILE_W)
         return rvhost::fail_msg(-3, "fused QKV epilogue: shape not taken");
     const Plan pl = plan_for(g.M, g.N, g.K);
     if (pl.splits < 2 || tune().reduce == 1) return rvhost::fail_msg(-3, "fused QKV epilogue: needs the split-K push form");
-    switch (pl.bn) {
-        case 16:
-            return dtype == 0 ? launch_one<16, EPI_QKV_ROPE, __half>(g, pl.splits, pl.stages, s, &rk)
-                              : launch_one<16, EPI_QKV_ROPE, __nv_bfloat16>(g, pl.splits, pl.stages, s, &rk);
-        case 32:
-            return dtype == 0 ? launch_one<32, EPI_QKV_ROPE, __half>(g, pl.splits, pl.stages, s, &rk)
-                              : launch_one<32, EPI_QKV_ROPE, __nv_bfloat16>(g, pl.splits, pl.stages, s, &rk);
-        case 64:  // (64- and 128-row tiles: the push goes into the peers' idle rings)
-            return dtype == 0 ? launch_one<64, EPI_QKV_ROPE, __half>(g, pl.splits, pl.stages, s, &rk)
-                              : launch_one<64, EPI_QKV_ROPE, __nv_bfloat16>(g, pl.splits, pl.stages, s, &rk);
-        default:
-            return dtype == 0 ? launch_one<128, EPI_QKV_ROPE, __half>(g, pl.splits, pl.stages, s, &rk)
-                              : launch_one<128, EPI_QKV_ROPE, __nv_bfloat16>(g, pl.splits, pl.stages, s, &rk);
-    }
+    if (pl.bn == 16)
+        return dtype == 0 ? launch_one<16, EPI_QKV_ROPE, __half>(g, pl.splits, pl.stages, s, &rk)
+                          : launch_one<16, EPI_QKV_ROPE, __nv_bfloat16>(g, pl.splits, pl.stages, s, &rk);
+    return dtype == 0 ? launch_one<32, EPI_QKV_ROPE, __half>(g, pl.splits, pl.stages, s, &rk)
+                      : launch_one<32, EPI_QKV_ROPE, __nv_bfloat16>(g, pl.splits, pl.stages, s, &rk);
 }
 
 // Residual GEMM whose activation operand is given as 16-bit values plus per-row partial maxima: the per-token
@@ -1273,20 +1192,12 @@ inline int launch_residual_a16(const TcArgs& g, int dtype, cudaStream_t s) {
 
 // LM head with the greedy argmax in the epilogue: per-tile winners into arg_val / arg_idx [M][ceil(N / 128)], then the
 // merge kernel.  Always an unsplit launch (a vocabulary-sized N has thousands of tiles; the plan would not split it).
-inline int launch_argmax(const TcArgs& g, int* out_tokens, cudaStream_t s) {
-    if (g.K % 16 != 0) return rvhost::fail_msg(-3, "tcgen05 GEMM needs K to be a multiple of 16");
-    Plan pl = plan_for(g.M, g.N, g.K);
-    pl.splits = 1;
-    pl.stages = tune().stages.load() > 0 ? tune().stages.load() : pick_stages(pl.bn, 1);
-    int rc;
-    switch (pl.bn) {
-        case 16: rc = launch_one<16, EPI_ARGMAX, __half>(g, 1, pl.stages, s); break;
-        case 32: rc = launch_one<32, EPI_ARGMAX, __half>(g, 1, pl.stages, s); break;
-        case 64: rc = launch_one<64, EPI_ARGMAX, __half>(g, 1, pl.stages, s); break;
-        case 128: rc = launch_one<128, EPI_ARGMAX, __half>(g, 1, pl.stages, s); break;
-        default: rc = launch_one<256, EPI_ARGMAX, __half>(g, 1, pl.stages, s); break;
-    }
-    if (rc) return rc;
+inline int launch_argmax(const TcArgs& g, cudaStream_t s) {
+    const Plan pl = plan_for(g.M, g.N, g.K);
+    const int stages = tune().stages.load() > 0 ? tune().stages.load() : pick_stages(pl.bn, 1);
+    return pl.bn == 16 ? launch_one<16, EPI_ARGMAX, __half>(g, 1, stages, s) : launch_one<32, EPI_ARGMAX, __half>(g, 1, stages, s);
+}
+inline int launch_argmax_merge(const TcArgs& g, int* out_tokens, cudaStream_t s) {
     const int tiles = (g.N + TILE_W - 1) / TILE_W;
     if (rv_launch(argmax_merge_kernel, dim3(g.M), dim3(256), 0, s, dim3(1, 1, 1), (const float*)g.arg_val, (const int*)g.arg_idx,
                   tiles, out_tokens) != cudaSuccess) {

@@ -1,0 +1,59 @@
+"""The CTA-pair GEMM (batches above 32 rows) at the edges of its tiles, against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from tests.test_gpu_gemm import TC, case, close, run  # noqa: E402
+
+
+# one row above the one-CTA form, tile widths 32..256 with remainders, one batch tile against two; weight rows that fill
+# no pair (200), end in the second CTA's half (1336) and a single K block up to split-K with uneven ranges
+@pytest.mark.parametrize("M", [33, 97, 128, 129, 255, 257, 513])
+@pytest.mark.parametrize("N,K", [(200, 64), (256, 512), (1336, 2176)])
+@pytest.mark.parametrize("mode", ["scale", "residual", "f32"])
+def test_pair_gemm(orc, M, N, K, mode):
+    a, a_s, w, w_s, cols, want = case(orc, M, N, K, seed=9)
+    dt = torch.float32 if mode == "f32" else torch.float16
+    res = None
+    if mode == "residual":
+        res = torch.from_numpy(np.random.default_rng(M).standard_normal((M, N)).astype(np.float32)).to(dt).cuda()
+    out = run(TC, a, a_s, w, w_s, dt, residual=res)
+    close(out.float().cpu().numpy(), want + (res.float().cpu().numpy() if res is not None else 0.0))
+
+
+# more tiles than pairs: the persistent loop, both accumulators, ring wrap-around
+@pytest.mark.parametrize("M,N,K", [(300, 43008, 576), (2048, 5376, 320), (8, 28672, 192)])
+def test_pair_gemm_many_tiles(orc, M, N, K):
+    a, a_s, w, w_s, cols, want = case(orc, M, N, K, seed=10, n_cols=64)
+    out = run(TC, a, a_s, w, w_s, torch.bfloat16)
+    close(out.float().cpu().numpy()[:, cols], want)
+
+
+@pytest.mark.parametrize("M", [33, 130, 300])
+@pytest.mark.parametrize("softcap", [0.0, 30.0])
+def test_pair_argmax_equals_argmax_over_logits(orc, M, softcap):
+    """The argmax epilogue against argmax over the same kernel's f32 logits, an all-NaN row and a tie included."""
+    from rvllm_b200 import _lib, gemm
+    from rvllm_b200.launchers import ArgmaxLaunch
+    V, K = 20008, 256
+    a, a_s, w, w_s, cols, want = case(orc, M, V, K, seed=11, n_cols=8)
+    d = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    A, W, AS, WS = d(a), d(w), d(a_s), d(w_s)
+    AS[1] = float("nan")
+    W[19000], WS[19000] = W[77], WS[77]  # the lower of two equal channels wins
+    L = _lib.lib()
+    ws = torch.empty(int(L.rvllm_fp8_gemm_lm_head_argmax_workspace(M, V)), dtype=torch.uint8, device="cuda")
+    tok = torch.empty(M, dtype=torch.int32, device="cuda")
+    assert L.rvllm_fp8_gemm_lm_head_argmax(tok.data_ptr(), A.data_ptr(), W.data_ptr(), AS.data_ptr(), WS.data_ptr(), M, V, K,
+                                           softcap, ws.data_ptr(), ws.numel(), _lib.current_stream()) == 0
+    logits = torch.empty((M, V), dtype=torch.float32, device="cuda")
+    gemm.fp8_gemm_channelscale(logits, A, W, AS, WS, impl=TC)
+    if softcap:
+        assert L.rvllm_logit_softcap_launch(logits.data_ptr(), M, V, softcap, 2, _lib.current_stream()) == 0
+    ref = torch.empty_like(tok)
+    ArgmaxLaunch(M, V).launch(logits, ref)
+    torch.cuda.synchronize()
+    assert gemm.tc_status() == 0
+    assert torch.equal(tok, ref) and int(tok[1]) == -1
