@@ -21,6 +21,7 @@
 #include "rowq_gemma.cu"
 #include "rowq_rmsnorm.cu"
 #include "rowq_silu.cu"
+#include "rowq_vec.cuh"
 
 namespace {
 
@@ -55,6 +56,39 @@ void rv_set_pdl(bool on) { g_pdl.store(on, std::memory_order_relaxed); }
 namespace rvhost {
 int fail_msg(int code, const char* msg) { return rv_fail(code, "%s", msg); }
 }  // namespace rvhost
+
+namespace {
+
+// Rows of up to 8192 values, 16-byte aligned, fit the registers of nt / 8 threads (norm_quant_vec_kernel).
+bool norm_vec_ok(uint32_t hidden, const void* out, const void* in, const void* gamma, const void* res_in, const void* res_out) {
+    return hidden <= 8192 && rv_aligned(out, 8) && rv_aligned(in, 16) && rv_aligned(gamma, 16) && rv_aligned(res_in, 16) &&
+           rv_aligned(res_out, 16);
+}
+template <typename T, bool RES>
+void launch_norm_vec(uint32_t tokens, uint32_t hidden, float eps, void* out, float* scale, void* res_out, const void* in,
+                     const void* res_in, const void* gamma, cudaStream_t s) {
+    const int nt = (int)round_block(rv_umin(hidden, 1024));  // the reference block whose order of summation is kept
+    const int per = nt / 8, nv = ((int)hidden / 8 + per - 1) / per;
+    const dim3 block((per + 31) / 32 * 32);
+    auto go = [&](auto kern) {
+        rv_launch(kern, dim3(tokens), block, 0, s, dim3(1, 1, 1), (uint8_t*)out, scale, (T*)res_out, (const T*)in, (const T*)res_in,
+                  (const T*)gamma, eps, (int)hidden, nt);
+    };
+    if (nv <= 2) go(rvrow::norm_quant_vec_kernel<T, 2, RES>);
+    else if (nv <= 4) go(rvrow::norm_quant_vec_kernel<T, 4, RES>);
+    else if (nv <= 6) go(rvrow::norm_quant_vec_kernel<T, 6, RES>);
+    else go(rvrow::norm_quant_vec_kernel<T, 8, RES>);
+}
+template <int ACT, typename T, int NC>
+int launch_act_stream(uint32_t rows, int inter, uint8_t* out, float* scale, const void* gate_up, cudaStream_t s) {
+    static RvDeviceOnce once;
+    auto kern = rvrow::act_mul_quant_stream_kernel<ACT, T, NC>;
+    if (rv_allow_smem(once, kern, 220 * 1024)) return -1;
+    rv_launch(kern, dim3(rv_umin(rows, 148)), dim3(1024), (size_t)8 * inter, s, dim3(1, 1, 1), out, scale, (const T*)gate_up, inter, (int)rows);
+    return 0;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -97,7 +131,12 @@ int rvllm_fused_rmsnorm_fp8_quant_launch(uint32_t num_tokens, uint32_t hidden, f
     if (dtype != RVLLM_F16 && dtype != RVLLM_BF16) return rv_fail(RVLLM_E_INVALID, "dtype must be f16 or bf16");
     dim3 grid(num_tokens), block(round_block(rv_umin(hidden, 1024)));
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == RVLLM_F16)
+    if (norm_vec_ok(hidden, out_fp8, in_hidden, gamma, nullptr, nullptr)) {
+        if (dtype == RVLLM_F16)
+            launch_norm_vec<__half, false>(num_tokens, hidden, eps, out_fp8, scale, nullptr, in_hidden, nullptr, gamma, s);
+        else
+            launch_norm_vec<__nv_bfloat16, false>(num_tokens, hidden, eps, out_fp8, scale, nullptr, in_hidden, nullptr, gamma, s);
+    } else if (dtype == RVLLM_F16)
         rv_launch(fused_rmsnorm_fp8_quant_kernel, dim3(grid), dim3(block), 128, s, dim3(1, 1, 1), (uint8_t*)out_fp8, scale, (const __half*)in_hidden,
                                                                 (const __half*)gamma, eps, (int)hidden);
     else
@@ -118,7 +157,12 @@ int rvllm_fused_add_rmsnorm_fp8_quant_launch(uint32_t num_tokens, uint32_t hidde
     if (dtype != RVLLM_F16 && dtype != RVLLM_BF16) return rv_fail(RVLLM_E_INVALID, "dtype must be f16 or bf16");
     dim3 grid(num_tokens), block(round_block(rv_umin(hidden, 1024)));
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == RVLLM_F16)
+    if (norm_vec_ok(hidden, out_fp8, in_hidden, gamma, residual_in, residual_out)) {
+        if (dtype == RVLLM_F16)
+            launch_norm_vec<__half, true>(num_tokens, hidden, eps, out_fp8, scale, residual_out, in_hidden, residual_in, gamma, s);
+        else
+            launch_norm_vec<__nv_bfloat16, true>(num_tokens, hidden, eps, out_fp8, scale, residual_out, in_hidden, residual_in, gamma, s);
+    } else if (dtype == RVLLM_F16)
         rv_launch(fused_add_rmsnorm_fp8_quant_kernel, dim3(grid), dim3(block), 128, s, dim3(1, 1, 1), 
             (uint8_t*)out_fp8, scale, (__half*)residual_out, (const __half*)in_hidden, (const __half*)residual_in,
             (const __half*)gamma, eps, (int)hidden);
@@ -144,7 +188,14 @@ int rvllm_quantize_fp8_per_token_launch(uint32_t num_tokens, uint32_t dim, void*
     if (dtype != RVLLM_F16 && dtype != RVLLM_BF16) return rv_fail(RVLLM_E_INVALID, "dtype must be f16 or bf16");
     dim3 grid(num_tokens), block(round_block(rv_umax(rv_umin(dim, 1024), 256)));
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == RVLLM_F16)
+    if (dim <= 32768 && rv_aligned(in, 16) && rv_aligned(out_fp8, 8)) {  // four vectors per thread hold the row
+        const dim3 vblock((dim / 8 + 127) / 128 * 32);
+        if (dtype == RVLLM_F16)
+            rv_launch(rvrow::quant_vec_kernel<__half>, grid, vblock, 0, s, dim3(1, 1, 1), (uint8_t*)out_fp8, scale, (const __half*)in, (int)dim);
+        else
+            rv_launch(rvrow::quant_vec_kernel<__nv_bfloat16>, grid, vblock, 0, s, dim3(1, 1, 1), (uint8_t*)out_fp8, scale,
+                      (const __nv_bfloat16*)in, (int)dim);
+    } else if (dtype == RVLLM_F16)
         rv_launch(quantize_fp8_per_token_kernel, dim3(grid), dim3(block), 128, s, dim3(1, 1, 1), (uint8_t*)out_fp8, scale, (const __half*)in, (int)dim);
     else
         rv_launch(quantize_fp8_per_token_bf16_kernel, dim3(grid), dim3(block), 128, s, dim3(1, 1, 1), (uint8_t*)out_fp8, scale,
@@ -197,6 +248,27 @@ int rvllm_fused_act_mul_fp8_quant_launch(uint32_t num_tokens, uint32_t intermedi
         else RV_ACT_CLUSTER(rvact::ACT_GELU, __nv_bfloat16);
 #undef RV_ACT_CLUSTER
         return rv_launched("fused_act_mul_fp8_quant (cluster)");
+    }
+    // Rows that do not fill 1024 threads with a vector each get as many warps as they have vectors; longer ones whose two
+    // buffers fit shared memory go through the persistent kernel (from about 100 rows on, see above).
+    block = dim3(rv_umin(1024u, (intermediate / 8 + 31) / 32 * 32));
+    if (intermediate > 8192 && 8u * intermediate <= 220u * 1024u) {
+        const bool nc3 = intermediate <= 3 * 8192;
+        int rc2;
+        if (act == RVLLM_ACT_SILU && dtype == RVLLM_F16)
+            rc2 = nc3 ? launch_act_stream<rvact::ACT_SILU, __half, 3>(num_tokens, I, o, scale, gate_up, s)
+                      : launch_act_stream<rvact::ACT_SILU, __half, 4>(num_tokens, I, o, scale, gate_up, s);
+        else if (act == RVLLM_ACT_SILU)
+            rc2 = nc3 ? launch_act_stream<rvact::ACT_SILU, __nv_bfloat16, 3>(num_tokens, I, o, scale, gate_up, s)
+                      : launch_act_stream<rvact::ACT_SILU, __nv_bfloat16, 4>(num_tokens, I, o, scale, gate_up, s);
+        else if (dtype == RVLLM_F16)
+            rc2 = nc3 ? launch_act_stream<rvact::ACT_GELU, __half, 3>(num_tokens, I, o, scale, gate_up, s)
+                      : launch_act_stream<rvact::ACT_GELU, __half, 4>(num_tokens, I, o, scale, gate_up, s);
+        else
+            rc2 = nc3 ? launch_act_stream<rvact::ACT_GELU, __nv_bfloat16, 3>(num_tokens, I, o, scale, gate_up, s)
+                      : launch_act_stream<rvact::ACT_GELU, __nv_bfloat16, 4>(num_tokens, I, o, scale, gate_up, s);
+        if (rc2) return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for the activation kernel");
+        return rv_launched("fused_act_mul_fp8_quant (stream)");
     }
     if (act == RVLLM_ACT_SILU && dtype == RVLLM_F16)
         rv_launch(fused_silu_mul_fp8_quant_kernel, dim3(grid), dim3(block), 128, s, dim3(1, 1, 1), o, scale, (const __half*)gate_up, I);
@@ -258,7 +330,27 @@ int rvllm_rope_fp8kv_launch(const void* q_in, const void* k_in, const void* v_in
     if (dtype != RVLLM_F16 && dtype != RVLLM_BF16) return rv_fail(RVLLM_E_INVALID, "dtype must be f16 or bf16");
     dim3 grid(num_tokens, num_heads > num_kv_heads ? num_heads : num_kv_heads), block(head_dim / 2);
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == RVLLM_F16)
+    // Vector form: head_dim / 8 lanes per head (512: / 16), operands aligned to a lane's vectors, whole vectors rotated.
+    const int ve = head_dim == 512 ? 8 : 4;
+    const bool pow2 = head_dim == 64 || head_dim == 128 || head_dim == 256 || head_dim == 512;
+    if (pow2 && num_tokens <= 65535 && (rotary_dim / 2) % ve == 0 && in_stride % ve == 0 && rv_aligned(q_in, 2 * ve) && rv_aligned(k_in, 2 * ve) &&
+        rv_aligned(v_in, 2 * ve) && rv_aligned(cos_table, 2 * ve) && rv_aligned(sin_table, 2 * ve) && rv_aligned(q_fp8, 4) &&
+        rv_aligned(k_cache, 4) && rv_aligned(v_cache, 4)) {
+        const int threads = (num_heads + 2 * num_kv_heads) * (head_dim / 2 / ve);
+        const dim3 vgrid((threads + 255) / 256, num_tokens);
+        auto go = [&](auto kern, auto tag) {
+            using T = decltype(tag);
+            rv_launch(kern, vgrid, dim3(256), 0, s, dim3(1, 1, 1), (const T*)q_in, (const T*)k_in, (const T*)v_in, in_stride,
+                      (uint8_t*)q_fp8, (uint8_t*)k_cache, (uint8_t*)v_cache, k_scale_cache, v_scale_cache, q_scale_cache,
+                      (const T*)cos_table, (const T*)sin_table, positions, slot_mapping, num_heads, num_kv_heads, head_dim,
+                      rotary_dim / 2, max_positions, num_cache_slots);
+        };
+        if (dtype == RVLLM_F16)
+            ve == 4 ? go(rvrow::rope_fp8kv_vec_kernel<__half, 4>, __half()) : go(rvrow::rope_fp8kv_vec_kernel<__half, 8>, __half());
+        else
+            ve == 4 ? go(rvrow::rope_fp8kv_vec_kernel<__nv_bfloat16, 4>, __nv_bfloat16())
+                    : go(rvrow::rope_fp8kv_vec_kernel<__nv_bfloat16, 8>, __nv_bfloat16());
+    } else if (dtype == RVLLM_F16)
         rv_launch(rvllm_rope_fp8kv_kernel, dim3(grid), dim3(block), 0, s, dim3(1, 1, 1), 
             (const __half*)q_in, (const __half*)k_in, (const __half*)v_in, in_stride, (uint8_t*)q_fp8,
             (uint8_t*)k_cache, (uint8_t*)v_cache, k_scale_cache, v_scale_cache, q_scale_cache,
