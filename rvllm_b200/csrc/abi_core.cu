@@ -50,7 +50,10 @@ int rv_launched(const char* what) {
     return RVLLM_OK;
 }
 static std::atomic<bool> g_pdl{true};
-bool rv_pdl_enabled() { return g_pdl.load(std::memory_order_relaxed); }
+static thread_local bool t_pdl = true;
+bool rv_pdl_enabled() { return t_pdl && g_pdl.load(std::memory_order_relaxed); }
+RvPdlScope::RvPdlScope(bool on) : before_(t_pdl) { t_pdl = on; }
+RvPdlScope::~RvPdlScope() { t_pdl = before_; }
 void rv_set_pdl(bool on) { g_pdl.store(on, std::memory_order_relaxed); }
 
 namespace rvhost {

@@ -147,6 +147,8 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
     return p != 0;
 }
+// Fetches a TMA descriptor ahead of its first use.
+__device__ __forceinline__ void prefetch_map(const void* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 // (the warp's number through a shuffle, so that the compiler knows it is the same in all lanes)
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 

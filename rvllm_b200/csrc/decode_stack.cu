@@ -124,8 +124,11 @@ struct rvllm_stack {
     cudaStream_t stream = nullptr;
     int skip_mask = 0;  // timing aid: launches left out of the step (rvllm_stack_debug_skip at creation time)
     bool capturing = false;  // enqueue_step is recording the graph (its kernels then run behind a complete predecessor step)
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    // One step, and a run of RUN_STEPS of them: a graph launch costs several microseconds between steps (a step of a small
+    // stack is 40), a kernel boundary inside a graph one or two.
+    static constexpr int RUN_STEPS = 8;
+    cudaGraph_t graph = nullptr, run_graph = nullptr;
+    cudaGraphExec_t exec = nullptr, run_exec = nullptr;
     int launches = 0;
     int steps_done = 0;
     int start_pos = 0;  // largest position any sequence had after the last reset / seeding (host-side copy)
@@ -303,7 +306,10 @@ int place_first_tokens(rvllm_stack* s) {
     return rv_launched("prepare_step");
 }
 
-int enqueue_step(rvllm_stack* s, int* launches) {
+// `chained`: the step follows another one inside the same graph.  Its first kernel is then launched without the
+// programmatic attribute: it starts when the step before has completed, so that the step's kernels may read the
+// bookkeeping early (see the attention launches) as they do at the start of a graph.
+int enqueue_step(rvllm_stack* s, int* launches, bool chained = false) {
     const int skip = s->skip_mask;
     auto on = [skip](int bit) { return (skip & bit) == 0; };
     const rvllm_stack_config& c = s->cfg;
@@ -312,7 +318,10 @@ int enqueue_step(rvllm_stack* s, int* launches) {
     int n = 0;
     // (slots, context lengths and block tables of this step were left by the previous step's advance_kernel, or by
     // reset / seeding: nothing below writes them)
-    RV_TRY(rvllm_embedding_gather_launch(s->residual, s->head.embedding, s->tokens, B, H, c.vocab, st));
+    {
+        const RvPdlScope scope(!chained);
+        RV_TRY(rvllm_embedding_gather_launch(s->residual, s->head.embedding, s->tokens, B, H, c.vocab, st));
+    }
     n++;
     // x_fp8 / x_scale hold the current layer's attention-block input (RMSNorm + quant of the residual) when the
     // previous layer's block kernel has already produced it
@@ -607,15 +616,19 @@ int rvllm_stack_create(rvllm_stack** out, const rvllm_stack_config* cfg, const r
     // are wiped by the reset below.
     if (rc == RVLLM_OK) rc = enqueue_step(s, &s->launches);
     if (rc == RVLLM_OK) rc = cuda_ok(cudaStreamSynchronize(s->stream), "eager warm-up step");
-    if (rc == RVLLM_OK) rc = cuda_ok(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-    if (rc == RVLLM_OK) {
+    auto record = [&](int steps, cudaGraph_t* graph, cudaGraphExec_t* exec) -> int {
+        RV_TRY(cuda_ok(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture"));
         s->capturing = true;
-        int rc2 = enqueue_step(s, nullptr);
+        int rc2 = RVLLM_OK;
+        for (int i = 0; i < steps && rc2 == RVLLM_OK; i++) rc2 = enqueue_step(s, nullptr, i > 0);
         s->capturing = false;
-        cudaError_t e = cudaStreamEndCapture(s->stream, &s->graph);
-        rc = rc2 != RVLLM_OK ? rc2 : cuda_ok(e, "end capture");
-    }
-    if (rc == RVLLM_OK) rc = cuda_ok(cudaGraphInstantiate(&s->exec, s->graph, 0), "graph instantiate");
+        const cudaError_t e = cudaStreamEndCapture(s->stream, graph);
+        RV_TRY(rc2);
+        RV_TRY(cuda_ok(e, "end capture"));
+        return cuda_ok(cudaGraphInstantiate(exec, *graph, 0), "graph instantiate");
+    };
+    if (rc == RVLLM_OK) rc = record(1, &s->graph, &s->exec);
+    if (rc == RVLLM_OK && cfg->max_context >= rvllm_stack::RUN_STEPS) rc = record(rvllm_stack::RUN_STEPS, &s->run_graph, &s->run_exec);
     if (rc == RVLLM_OK) rc = rvllm_stack_reset(s, nullptr);
     if (rc != RVLLM_OK) {
         rvllm_stack_destroy(s);
@@ -628,8 +641,10 @@ int rvllm_stack_create(rvllm_stack** out, const rvllm_stack_config* cfg, const r
 void rvllm_stack_destroy(rvllm_stack* s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    if (s->exec) cudaGraphExecDestroy(s->exec);
-    if (s->graph) cudaGraphDestroy(s->graph);
+    for (cudaGraphExec_t e : {s->exec, s->run_exec})
+        if (e) cudaGraphExecDestroy(e);
+    for (cudaGraph_t g : {s->graph, s->run_graph})
+        if (g) cudaGraphDestroy(g);
     if (s->pinned) cudaFreeHost(s->pinned);
     if (s->arena) cudaFree(s->arena);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -719,7 +734,11 @@ static int room_for(rvllm_stack* s, int n) {
 int rvllm_stack_run(rvllm_stack* s, int n) {
     if (!s || n < 0) return rv_fail(RVLLM_E_INVALID, "bad run arguments");
     RV_TRY(room_for(s, n));
-    for (int i = 0; i < n; i++) RV_TRY(cuda_ok(cudaGraphLaunch(s->exec, s->stream), "graph launch"));
+    for (int left = n; left > 0;) {
+        const bool many = s->run_exec && left >= rvllm_stack::RUN_STEPS;
+        RV_TRY(cuda_ok(cudaGraphLaunch(many ? s->run_exec : s->exec, s->stream), "graph launch"));
+        left -= many ? rvllm_stack::RUN_STEPS : 1;
+    }
     s->steps_done += n;
     return RVLLM_OK;
 }

@@ -136,6 +136,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     const int set_cols = p.npart * BN;
 
     if (threadIdx.x == 0) {
+        rv::prefetch_map(&map_w);
+        rv::prefetch_map(&map_a);
         for (int s = 0; s < STAGES; s++) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);

@@ -299,6 +299,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     rv::pdl_launch();
     if (threadIdx.x == 0) {
         trace_point(p.trace, 0);  // the CTA runs
+        rv::prefetch_map(&map_w);
+        if (!A16) rv::prefetch_map(&map_a);
         for (int s = 0; s < STAGES; s++) {
             mbar_init(full + s, A16 ? 5 : 1);  // the producer's arrival (+ one per converting warp)
             mbar_init(empty + s, 1);

@@ -16,6 +16,16 @@ inline uint32_t rv_umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 // Whether launches carry the programmatic-stream-serialization attribute (on by default).
 bool rv_pdl_enabled();
 void rv_set_pdl(bool on);
+// While it lives, launches of the calling thread carry the attribute only if `on` and the process-wide switch say so.
+struct RvPdlScope {
+    explicit RvPdlScope(bool on);
+    ~RvPdlScope();
+    RvPdlScope(const RvPdlScope&) = delete;
+    RvPdlScope& operator=(const RvPdlScope&) = delete;
+
+  private:
+    bool before_;
+};
 
 // Launch with optional cluster dimensions and, when enabled, programmatic dependent launch.
 template <typename... KArgs, typename... Args>

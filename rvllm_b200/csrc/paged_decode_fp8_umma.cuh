@@ -235,6 +235,8 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
 
     // ---- set-up that does not depend on the preceding kernel ----
     if (tid == 0) {
+        rv::prefetch_map(&map_k);
+        rv::prefetch_map(&map_v);
         for (int i = 0; i < NUNITS; i++) {
             mbar_init(full + i, 1);
             mbar_init(empty + i, 1);
