@@ -244,13 +244,14 @@ int rvllm_paged_decode_fp8_validate(int batch_size, int num_heads, int num_kv_he
                                     int window_size_left, float scale);
 uint64_t rvllm_paged_decode_workspace_size(int batch_size, int num_heads, int num_kv_heads, int head_dim);
 int rvllm_paged_decode_max_chunks(int batch_size, int num_kv_heads);
-/* Variant 4 is the tcgen05 / TMA main kernel (head_dim 128 or 256, at most 8 query heads per KV
+/* Variant 4 is the tcgen05 / TMA main kernel (head_dim 128, 256 or 512, at most 8 query heads per KV
  * head, pages of 8..128 tokens that divide 128).  Its waits on mbarriers are bounded; this reads
  * (and optionally clears) the word that records the first wait that gave up: 0 = none. */
 int rvllm_paged_decode_tc_status(int* status, int reset);
 /* Which main kernel a launch of this shape runs (1 = both products on the FP32 pipes, 2 = scores on
  * mma.sync FP8 tensor cores and P.V on the FP32 pipes, 3 = both products on mma.sync, 4 = tcgen05 /
- * TMEM / TMA: 4 where the shape allows it, else 3, else 2); negative on bad arguments. */
+ * TMEM / TMA: 4 where the shape allows it, else 3, else 2); negative on bad arguments.  head_dim 512 is reported as 2
+ * although its plain form runs on 4: it leaves no per-KV-head maxima, which is what callers ask this for. */
 int rvllm_paged_decode_kernel_for(int num_heads, int num_kv_heads, int head_dim, int block_size, int num_blocks_total);
 int rvllm_paged_decode_fp8(const void* q_fp8, const void* k_cache_fp8, const void* v_cache_fp8, void* output,
                            int out_dtype, const int32_t* block_tables, const int32_t* context_lens,

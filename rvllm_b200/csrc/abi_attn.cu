@@ -20,9 +20,7 @@ static std::atomic<int> g_cluster_combine{1};
 static std::atomic<int> g_early_meta{0};       // 0: when the caller hinted it (below), 1: always, -1: never
 static thread_local int t_early_meta_once = 0;  // one-shot hint of the calling thread, taken by its next launch
 static std::atomic<int> g_cluster_min_tokens{rvua::TOK};  // smallest chunk of the cluster-merged split-KV form
-// CTAs the cluster-merged form aims for: chunks cost it neither workspace traffic nor a second launch
-constexpr int CLUSTER_TARGET_CTAS = rvattn::TARGET_CTAS;
-static std::atomic<int> g_cluster_target{CLUSTER_TARGET_CTAS};
+static std::atomic<int> g_cluster_target{0};  // CTAs the cluster-merged form aims for, 0 = rvua::pick_cluster_chunks
 static std::atomic<int> g_ring_units{0};  // tcgen05 kernel: K/V ring depth in 16 KB units, 0 = automatic
 static std::atomic<int> g_variant{0};  // 0 automatic (tcgen05 kernel where the shape allows, else 3, else 2), 1 FP32-pipe kernel,
                            // 2 mma.sync scores + FP32-pipe P.V, 3 both products on mma.sync, 4 tcgen05 / TMA
@@ -93,7 +91,7 @@ void rvllm_paged_decode_early_meta(int mode) { g_early_meta = mode > 0 ? 1 : (mo
 void rvllm_paged_decode_hint_early_meta(void) { t_early_meta_once = 1; }
 void rvllm_paged_decode_cluster_combine(int enabled) { g_cluster_combine = enabled != 0; }
 void rvllm_paged_decode_cluster_tune(int target_ctas, int min_chunk_tokens) {
-    g_cluster_target = target_ctas > 0 ? target_ctas : CLUSTER_TARGET_CTAS;
+    g_cluster_target = target_ctas > 0 ? target_ctas : 0;
     g_cluster_min_tokens = min_chunk_tokens > 0 ? min_chunk_tokens : rvua::TOK;
 }
 
@@ -121,34 +119,30 @@ struct QuantOut {
     float* amax = nullptr;   // when set (tcgen05 kernel, one chunk): max |stored output| per (sequence, kv_head)
 };
 
-// tcgen05 / TMA main kernel (head_dim 128 or 256, up to 8 query heads per KV head)
+// tcgen05 / TMA main kernel (head_dim 128, 256 or 512, up to 8 query heads per KV head)
 template <int HD, int GT, typename OutT, bool CL>
 int launch_umma_form(const rvattn::Params& p, cudaStream_t s) {
-    if constexpr (HD == 128 || HD == 256) {
-        CUtensorMap mk, mv;
-        const long long slots = (long long)p.num_blocks_total * p.block_size;
-        if (!rvua::cache_map(&mk, p.k_cache, slots, p.kv_heads, HD, p.block_size) ||
-            !rvua::cache_map(&mv, p.v_cache, slots, p.kv_heads, HD, p.block_size))
-            return rv_fail(RVLLM_E_LAUNCH, "cuTensorMapEncodeTiled failed for the KV cache");
-        auto kern = rvua::paged_decode_fp8_umma_kernel<HD, GT, OutT, CL>;
-        using C = rvua::Cfg<HD>;
-        static RvDeviceOnce smem_once;  // per kernel instantiation and device
-        if (rv_allow_smem(smem_once, kern, C::smem_bytes(rvua::MAX_UNITS)))
-            return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
-        const int ring = g_ring_units.load();
-        // cluster-combine form: the chunks of a (sequence, KV head) are one cluster, the receive area sits behind the rest
-        // (and counts when the ring depth is chosen: a third of the footprint at eight chunks)
-        const size_t recv = p.cluster_combine ? (size_t)C::recv_bytes(p.max_chunks, p.heads / p.kv_heads) : 0;
-        int units = ring > 0 ? ring : rvua::pick_units<HD>((long long)p.kv_heads * p.max_chunks * p.batch, (int)recv);
-        if (units < C::MIN_UNITS) units = C::MIN_UNITS;
-        if (units > rvua::MAX_UNITS) units = rvua::MAX_UNITS;
-        while (units > C::MIN_UNITS && C::smem_bytes(units) + recv > (size_t)C::smem_bytes(rvua::MAX_UNITS)) units--;
-        rv_launch(kern, dim3(p.kv_heads, p.max_chunks, p.batch), dim3(rvua::THREADS), (size_t)C::smem_bytes(units) + recv, s,
-                  dim3(1, p.cluster_combine ? p.max_chunks : 1, 1), mk, mv, p, units);
-        return rv_launched("paged_decode_fp8 (tcgen05)");
-    } else {
-        return rv_fail(RVLLM_E_UNSUPPORTED, "tcgen05 decode attention needs head_dim 128 or 256");
-    }
+    CUtensorMap mk, mv;
+    const long long slots = (long long)p.num_blocks_total * p.block_size;
+    if (!rvua::cache_map(&mk, p.k_cache, slots, p.kv_heads, HD, p.block_size) ||
+        !rvua::cache_map(&mv, p.v_cache, slots, p.kv_heads, HD, p.block_size))
+        return rv_fail(RVLLM_E_LAUNCH, "cuTensorMapEncodeTiled failed for the KV cache");
+    auto kern = rvua::paged_decode_fp8_umma_kernel<HD, GT, OutT, CL>;
+    using C = rvua::Cfg<HD>;
+    static RvDeviceOnce smem_once;  // per kernel instantiation and device
+    if (rv_allow_smem(smem_once, kern, C::smem_bytes(C::MOST_UNITS)))
+        return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
+    const int ring = g_ring_units.load();
+    // cluster-combine form: the chunks of a (sequence, KV head) are one cluster, the receive area sits behind the rest
+    // (and counts when the ring depth is chosen: a third of the footprint at eight chunks)
+    const size_t recv = p.cluster_combine ? (size_t)C::recv_bytes(p.max_chunks, p.heads / p.kv_heads) : 0;
+    int units = ring > 0 ? ring : rvua::pick_units<HD>((long long)p.kv_heads * p.max_chunks * p.batch, (int)recv);
+    if (units < C::MIN_UNITS) units = C::MIN_UNITS;
+    if (units > C::MOST_UNITS) units = C::MOST_UNITS;
+    while (units > C::MIN_UNITS && C::smem_bytes(units) + recv > (size_t)C::smem_bytes(C::MOST_UNITS)) units--;
+    rv_launch(kern, dim3(p.kv_heads, p.max_chunks, p.batch), dim3(rvua::THREADS), (size_t)C::smem_bytes(units) + recv, s,
+              dim3(1, p.cluster_combine ? p.max_chunks : 1, 1), mk, mv, p, units);
+    return rv_launched("paged_decode_fp8 (tcgen05)");
 }
 
 template <int HD, int GT, typename OutT>
@@ -156,17 +150,23 @@ int launch_umma(const rvattn::Params& p, cudaStream_t s) {
     return p.cluster_combine ? launch_umma_form<HD, GT, OutT, true>(p, s) : launch_umma_form<HD, GT, OutT, false>(p, s);
 }
 
+bool takes_umma(const rvattn::Params& p, int head_dim, bool amax) {
+    if (g_variant != 4 && g_variant != 0) return false;
+    return rvua::supports(p, head_dim) || (!amax && rvua::supports_wide(p, head_dim));
+}
+
 template <int HD, int GT, typename OutT>
 int launch_main(const rvattn::Params& p, cudaStream_t s) {
-    dim3 grid(p.kv_heads, p.max_chunks, p.batch);
-    if ((g_variant == 4 || g_variant == 0) && rvua::supports(p, HD)) {
+    if constexpr (HD >= 128) {
+        if (!takes_umma(p, HD, p.amax_out != nullptr)) return 1;  // not handled here
         const int group = p.heads / p.kv_heads;
         if (group <= 1) return launch_umma<HD, 1, OutT>(p, s);
         if (group <= 2) return launch_umma<HD, 2, OutT>(p, s);
         if (group <= 4) return launch_umma<HD, 4, OutT>(p, s);
         return launch_umma<HD, 8, OutT>(p, s);
+    } else {
+        return 1;
     }
-    return 1;  // not handled here
 }
 
 template <int HD, int GT, typename OutT>
@@ -304,21 +304,27 @@ static int decode_core(const QuantOut& qo, const void* q_fp8, const void* k_cach
         t_early_meta_once = 0;
         p.early_meta = mode > 0 || (mode == 0 && hinted);
     }
-    const bool umma = (g_variant == 4 || g_variant == 0) && rvua::supports(p, head_dim);
-    const int cchunks = rvattn::pick_max_chunks(batch_size, num_kv_heads, g_cluster_target);
-    if (umma && cchunks > 1 && !qo.fp8 && g_cluster_combine.load() != 0) {
+    const bool umma = takes_umma(p, head_dim, qo.amax != nullptr);
+    if (umma && !qo.fp8 && g_cluster_combine.load() != 0) {
         // Split-KV without the workspace round trip and the combine launch: up to 8 chunks of at least one
         // 128-token tile, one thread-block cluster per (sequence, KV head), merged in the chunk-0 CTA.
-        int cc = cchunks < 8 ? cchunks : 8;
         const int group = num_heads / num_kv_heads;
-        while (cc > 1 && cc * group * (head_dim + 2) * 4 > rvua::MAX_RECV_BYTES) cc--;
-        if (cc > 1) {
-            p.max_chunks = cc;
-            p.min_chunk_tokens = g_cluster_min_tokens.load();
-            p.cluster_combine = 1;
+        int cc;
+        if (g_cluster_target.load() > 0) {  // a tuning run's own target
+            cc = rvattn::pick_max_chunks(batch_size, num_kv_heads, g_cluster_target);
+            if (cc > 8) cc = 8;
+            while (cc > 1 && cc * group * (head_dim + 2) * 4 > rvua::MAX_RECV_BYTES) cc--;
+        } else {
+            // tokens a sequence can attend: its block table's capacity, or the window
+            long long len = (long long)block_size * max_blocks_per_seq;
+            if (window_size_left >= 0 && window_size_left + 1ll < len) len = window_size_left + 1ll;
+            cc = rvua::pick_cluster_chunks((long long)batch_size * num_kv_heads, (int)(len < (1 << 20) ? len : (1 << 20)), group, head_dim);
         }
+        p.max_chunks = cc;
+        p.min_chunk_tokens = g_cluster_min_tokens.load();
+        p.cluster_combine = cc > 1;
     }
-    if (qo.amax && !(umma && (chunks == 1 || p.cluster_combine)))
+    if (qo.amax && !(umma && (p.max_chunks == 1 || p.cluster_combine)))
         return rv_fail(RVLLM_E_UNSUPPORTED, "the per-token absmax output needs the tcgen05 kernel with one chunk or the cluster merge");
     cudaStream_t s = (cudaStream_t)stream;
     return out_dtype == RVLLM_F16 ? launch_attn_hd<__half>(p, qo, head_dim, s)

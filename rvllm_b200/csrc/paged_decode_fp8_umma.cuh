@@ -172,12 +172,13 @@ __host__ __device__ constexpr uint32_t instr_desc(int n, bool a_mn) {
     return (1u << 4) | (a_mn ? (1u << 15) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-constexpr int MAX_UNITS = 8;
+constexpr int MAX_UNITS = 12;
 template <int HD> struct Cfg {
     static constexpr int HALVES = HD / PANEL;            // 128-byte panels per K or V tile
     static constexpr int UPT = 2 * HALVES;               // ring units per tile: K panels, then V panels
-    static constexpr int MIN_UNITS = HALVES == 1 ? 2 : 3;     // both K panels plus one more must fit
-    static constexpr int TMEM_COLS = HALVES == 1 ? 64 : 128;  // scores 2 x 16, then HALVES x 32 accumulator columns
+    static constexpr int MIN_UNITS = HALVES + 1;         // all K panels plus one more must fit
+    static constexpr int MOST_UNITS = HALVES == 4 ? MAX_UNITS : 8;
+    static constexpr int TMEM_COLS = HALVES == 1 ? 64 : HALVES == 2 ? 128 : 256;  // scores 2 x 16, then HALVES x 32 accumulator columns
     static constexpr int O_COL = 32;
     static constexpr int P_BYTES = NP * PANEL;           // 4 KB
     static constexpr int Q_BYTES = HALVES * NQ * PANEL;  // 2 KB per panel
@@ -203,7 +204,7 @@ template <int HD, int GT, typename OutT, bool CL>
 __global__ void __launch_bounds__(THREADS, 1)
 paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, Params p,
                              int nunits) {
-    static_assert(HD == 128 || HD == 256, "one or two 128-byte panels per cache row");
+    static_assert(HD == 128 || HD == 256 || HD == 512, "one, two or four 128-byte panels per cache row");
     static_assert(GT >= 1 && GT <= 8, "up to 8 query heads share the score tile");
     using C = Cfg<HD>;
     constexpr int HALVES = C::HALVES, UPT = C::UPT;
@@ -286,14 +287,15 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
         if (chunk >= nchunks) {
             active = false;
         } else {
-            const int chunk_size = (len + nchunks - 1) / nchunks;
+            int chunk_size = (len + nchunks - 1) / nchunks;
+            if (CL) chunk_size = (chunk_size + TOK - 1) / TOK * TOK;  // whole tiles (1143 tokens are nine or ten)
             t_begin = start + chunk * chunk_size;
             t_end = min(t_begin + chunk_size, start + len);
         }
     }
     const int bs = p.block_size;
     const int tile0 = active ? (t_begin / bs) * bs : 0;              // first tile starts on a page boundary
-    const int ntiles = active ? (t_end - tile0 + TOK - 1) / TOK : 0;
+    const int ntiles = active && t_end > t_begin ? (t_end - tile0 + TOK - 1) / TOK : 0;
     const int* table = p.block_tables + (size_t)b * p.max_blocks_per_seq;
 
     tc_fence_before();
@@ -684,7 +686,7 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
         // partial or not — arrives (release, cluster scope) on chunk 0's mbarrier after its stores; chunk 0 waits for
         // all of them; the others are done.
         if (chunk != 0 && warp >= 2) {
-            if (active && nchunks > 1) {
+            if (ntiles > 0 && nchunks > 1) {
                 bar_softmax();  // the staged partial is complete
                 const uint32_t dst = smem_u32(recv + (size_t)chunk * nh * PSTRIDE);
                 for (int i = tid - 64; i < nh * PSTRIDE; i += 128) st_cluster_f32(dst + (uint32_t)i * 4u, 0u, recv[i]);
@@ -723,7 +725,7 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
             const int row = (warp - 2) * 32 + lane;
             int m_start, m_len;
             rvattn::attend_interval(ctx, p.window_size_left, m_start, m_len);
-            const int m_size = (m_len + nchunks - 1) / nchunks;
+            const int m_size = ((m_len + nchunks - 1) / nchunks + TOK - 1) / TOK * TOK;
             float amax = 0.0f;
 #pragma unroll
             for (int h = 0; h < HALVES; h++) {
@@ -816,11 +818,14 @@ inline bool cache_map(CUtensorMap* out, const void* base, long long slots, int k
 
 // Shapes this kernel takes: head_dim 128 or 256, at most 8 query heads per KV head, pages of 8..128
 // tokens that tile 128, 16-byte aligned caches.
-inline bool supports(const Params& p, int head_dim) {
-    const int group = p.heads / p.kv_heads;
-    return (head_dim == 128 || head_dim == 256) && group <= 8 && p.block_size >= 8 && p.block_size <= TOK &&
-           TOK % p.block_size == 0 && (long long)p.num_blocks_total * p.block_size < (1ll << 31);
+inline bool heads_and_pages_ok(const Params& p) {
+    return p.heads / p.kv_heads <= 8 && p.block_size >= 8 && p.block_size <= TOK && TOK % p.block_size == 0 &&
+           (long long)p.num_blocks_total * p.block_size < (1ll << 31);
 }
+inline bool supports(const Params& p, int head_dim) { return (head_dim == 128 || head_dim == 256) && heads_and_pages_ok(p); }
+// And, for plain outputs (no per-KV-head maxima), head_dim 512: one CTA per SM of 12 ring units (10 sequences of up to 3000
+// tokens, 32 / 16 heads: 222 us on the mma.sync form, 89 here).
+inline bool supports_wide(const Params& p, int head_dim) { return head_dim == 512 && heads_and_pages_ok(p); }
 
 // Ring depth.  A shallow ring lets more CTAs share an SM (the footprint is 8-10 KB + 16 KB per unit), a
 // deep one lets a CTA run further ahead of its softmax.  The choice minimises
@@ -834,7 +839,8 @@ template <int HD> inline int pick_units(long long ctas, int extra_bytes = 0) {
     };
     static const Cand c128[] = {{2, 1.25}, {3, 1.0}, {4, 0.87}, {6, 0.74}};
     static const Cand c256[] = {{4, 1.15}, {6, 1.0}};
-    const Cand* cand = C::HALVES == 1 ? c128 : c256;
+    static const Cand c512[] = {{6, 1.15}, {12, 1.0}};
+    const Cand* cand = C::HALVES == 1 ? c128 : C::HALVES == 2 ? c256 : c512;
     const int n = C::HALVES == 1 ? 4 : 2;
     int best = cand[0].units;
     double best_cost = 1e300;
@@ -844,6 +850,36 @@ template <int HD> inline int pick_units(long long ctas, int extra_bytes = 0) {
         if (cost < best_cost) {
             best_cost = cost;
             best = cand[i].units;
+        }
+    }
+    return best;
+}
+
+// Chunks per sequence of the cluster-merged form (1: no split, no cluster) for `units` (sequence, KV head) pairs that attend
+// up to `len` tokens: the cheapest of 1 to 8, in tiles of one CTA.  A CTA is a chain of about 1.5 us per tile with a few
+// CTAs per SM, plus about two tiles of prologue and one of merging.  Half of the cost is what equal contexts take
+// (waves x chunk), half what contexts spread up to `len` take (the mean load of a residency slot and the tail of the
+// longest chunk).  Residency: registers allow 4 / 3 / 2 CTAs of up to 2 / 4 / 8 query heads, the ring 2 and 1 at head_dim
+// 256 and 512.  Measured, us, with the fixed target of 296 CTAs this replaces -> now: 64 sequences of 512 to 32768 tokens,
+// head_dim 256: 1512 -> 1373; 8 of them, head_dim 128: 148 -> 118; 16 of up to 4000 tokens, 64 / 8 heads: 45 -> 33;
+// 4 of up to 100 tokens (no cluster at all now): 6.9 -> 5.2.
+inline int pick_cluster_chunks(long long units, int len, int heads_per_cta, int head_dim) {
+    int per_sm = heads_per_cta <= 2 ? 4 : heads_per_cta <= 4 ? 3 : 2;
+    if (head_dim == 256 && per_sm > 2) per_sm = 2;
+    if (head_dim == 512) per_sm = 1;
+    const long long slots = 148ll * per_sm;
+    const int tiles = (len + TOK - 1) / TOK;
+    int best = 1;
+    double best_cost = 1e300;
+    for (int cc = 1; cc <= 8 && cc <= tiles; cc++) {
+        if (cc > 1 && cc * heads_per_cta * (head_dim + 2) * 4 > MAX_RECV_BYTES) break;
+        const int fixed = cc > 1 ? 3 : 2;
+        const double chunk = (tiles + cc - 1) / cc + fixed;
+        const double even = (double)((units * cc + slots - 1) / slots) * chunk;
+        const double spread = (double)units * (0.6 * tiles + cc * fixed) / slots + 0.5 * chunk;
+        if (even + spread < best_cost) {
+            best_cost = even + spread;
+            best = cc;
         }
     }
     return best;
