@@ -304,9 +304,9 @@ int rvllm_argmax_launch(uint32_t num_tokens, uint32_t vocab, const float* logits
         dim3 grid((vocab + 1023) / 1024, num_tokens), block(256);
         rv_launch(argmax_grid_f32_kernel, dim3(grid), dim3(block), 0, s, dim3(1, 1, 1), logits, out, (int)vocab);
     } else if (vocab >= 32768 && num_tokens <= 192) {
-        // few long rows: eight CTAs per row (same winner, see greedy_argmax_cluster.cuh); 1024 threads while
-        // two such CTAs per SM hold the whole grid, 512 beyond (four per SM)
-        dim3 cgrid(8, num_tokens), cblock(num_tokens <= 32 ? rvargmax::ARGMAX_CLUSTER_THREADS : 512), cdim(8, 1, 1);
+        // few long rows: eight CTAs per row (same winner, see greedy_argmax_cluster.cuh); 256 threads with eight vectors in
+        // flight each, five such CTAs per SM hold the grids of up to 92 rows at once
+        dim3 cgrid(8, num_tokens), cblock(rvargmax::ARGMAX_CLUSTER_THREADS), cdim(8, 1, 1);
         rv_launch(rvargmax::argmax_cluster_f32_kernel, cgrid, cblock, 0, s, cdim, logits, out, (int)vocab);
     } else {
         uint32_t b = 1;
@@ -333,12 +333,18 @@ int rvllm_rope_fp8kv_launch(const void* q_in, const void* k_in, const void* v_in
     if (dtype != RVLLM_F16 && dtype != RVLLM_BF16) return rv_fail(RVLLM_E_INVALID, "dtype must be f16 or bf16");
     dim3 grid(num_tokens, num_heads > num_kv_heads ? num_heads : num_kv_heads), block(head_dim / 2);
     cudaStream_t s = (cudaStream_t)stream;
-    // Vector form: head_dim / 8 lanes per head (512: / 16), operands aligned to a lane's vectors, whole vectors rotated.
-    const int ve = head_dim == 512 ? 8 : 4;
+    // Vector form: operands aligned to a lane's VE elements, whole vectors rotated.  VE = 4 (head_dim / 8 lanes per head)
+    // for few tokens, where threads are short, VE = 8 for many heads of 128 or more (1000 tokens of 64 heads of 128:
+    // 10.5 -> 7.4 us; heads of 64: 8.6 -> 9.7) and at head_dim 512, whose 64 lanes are no warp.
     const bool pow2 = head_dim == 64 || head_dim == 128 || head_dim == 256 || head_dim == 512;
-    if (pow2 && num_tokens <= 65535 && (rotary_dim / 2) % ve == 0 && in_stride % ve == 0 && rv_aligned(q_in, 2 * ve) && rv_aligned(k_in, 2 * ve) &&
-        rv_aligned(v_in, 2 * ve) && rv_aligned(cos_table, 2 * ve) && rv_aligned(sin_table, 2 * ve) && rv_aligned(q_fp8, 4) &&
-        rv_aligned(k_cache, 4) && rv_aligned(v_cache, 4)) {
+    auto vec_ok = [&](int ve) {
+        return pow2 && num_tokens <= 65535 && (rotary_dim / 2) % ve == 0 && in_stride % ve == 0 && rv_aligned(q_in, 2 * ve) &&
+               rv_aligned(k_in, 2 * ve) && rv_aligned(v_in, 2 * ve) && rv_aligned(cos_table, 2 * ve) && rv_aligned(sin_table, 2 * ve) &&
+               rv_aligned(q_fp8, ve) && rv_aligned(k_cache, ve) && rv_aligned(v_cache, ve);
+    };
+    const bool many = head_dim >= 128 && (long long)num_tokens * (num_heads + 2 * num_kv_heads) * head_dim >= (1ll << 20);
+    const int ve = (head_dim == 512 || many) && vec_ok(8) ? 8 : 4;
+    if (vec_ok(ve) && head_dim / 2 / ve <= 32) {
         const int threads = (num_heads + 2 * num_kv_heads) * (head_dim / 2 / ve);
         const dim3 vgrid((threads + 255) / 256, num_tokens);
         auto go = [&](auto kern, auto tag) {

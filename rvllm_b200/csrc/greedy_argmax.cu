@@ -63,7 +63,7 @@ __device__ __forceinline__ bool launch_ok(int vocab) {
 }
 
 // scan x[begin, end) of one row; indices reported relative to the row start
-__device__ __forceinline__ Cand scan_f32(const float* __restrict__ x, long long begin, long long end) {
+__device__ __forceinline__ Cand scan_f32(const float* x, long long begin, long long end) {
     Cand b;
     b.v = -CUDART_INF_F;
     b.i = -1;
@@ -101,9 +101,59 @@ __device__ __forceinline__ Cand scan_f32(const float* __restrict__ x, long long 
     return b;
 }
 
+// The same scan with one comparison and two selects per element: a strict "greater" with a running best per component of
+// the vectors, eight vectors in flight (out-of-range ones read as -inf).  It passes over -inf, which may only win a row
+// without anything greater: row_best() falls back to scan_f32 then.
+__device__ __forceinline__ Cand scan_f32_above(const float* x, long long begin, long long end) {
+    constexpr int U = 8;
+    Cand b;
+    b.v = -CUDART_INF_F;
+    b.i = -1;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const long long peel = ((16 - (reinterpret_cast<uintptr_t>(x + begin) & 15)) & 15) >> 2;
+    const long long head = begin + peel < end ? begin + peel : end;
+    for (long long i = begin + tid; i < head; i += nt) take(b, x[i], (int)i);
+    const int nvec = (int)((end - head) >> 2);
+    const float4* xv = reinterpret_cast<const float4*>(x + head);
+    float best[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+    int at[4] = {-1, -1, -1, -1};
+    for (int v0 = tid; v0 < nvec; v0 += U * nt) {
+        float4 q[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const int v = v0 + k * nt;
+            q[k] = v < nvec ? __ldcs(xv + v) : make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const float* f = &q[k].x;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const bool more = f[c] > best[c];
+                best[c] = more ? f[c] : best[c];
+                at[c] = more ? v0 + k * nt : at[c];
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        if (at[c] >= 0) take(b, best[c], (int)head + 4 * at[c] + c);
+    for (long long i = head + 4ll * nvec + tid; i < end; i += nt) take(b, x[i], (int)i);
+    return b;
+}
+// The block's winner over x[begin, end); every thread returns it.
+__device__ __forceinline__ Cand row_best(const float* x, long long begin, long long end, float* sv, int* si) {
+    Cand b = block_best(scan_f32_above(x, begin, end), sv, si);
+    if (b.i < 0 || b.v == -CUDART_INF_F) {  // nothing above -inf (block-uniform)
+        __syncthreads();
+        b = block_best(scan_f32(x, begin, end), sv, si);
+    }
+    return b;
+}
+
 }  // namespace
 
-extern "C" __global__ void argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab) {
+extern "C" __global__ void argmax_kernel(const float* logits, int* __restrict__ out, int vocab) {
     __shared__ float sv[32];
     __shared__ int si[32];
     rv::pdl_launch();
@@ -113,8 +163,7 @@ extern "C" __global__ void argmax_kernel(const float* __restrict__ logits, int* 
         if (out != nullptr && threadIdx.x == 0) out[row] = -1;
         return;
     }
-    Cand b = scan_f32(logits + (long long)row * vocab, 0, vocab);
-    b = block_best(b, sv, si);
+    const Cand b = row_best(logits + (long long)row * vocab, 0, vocab, sv, si);
     if (threadIdx.x == 0) out[row] = b.i;
 }
 
@@ -137,7 +186,7 @@ extern "C" __global__ void argmax_f16_kernel(const __half* __restrict__ logits, 
     if (threadIdx.x == 0) out[row] = b.i;
 }
 
-extern "C" __global__ void argmax_grid_f32_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab) {
+extern "C" __global__ void argmax_grid_f32_kernel(const float* logits, int* __restrict__ out, int vocab) {
     __shared__ float sv[32];
     __shared__ int si[32];
     rv::pdl_launch();
@@ -148,8 +197,7 @@ extern "C" __global__ void argmax_grid_f32_kernel(const float* __restrict__ logi
     const long long begin = (long long)blockIdx.x * chunk;
     const long long end = begin + chunk < vocab ? begin + chunk : vocab;
     const float* x = logits + (long long)row * vocab;
-    Cand b = scan_f32(x, begin < end ? begin : end, end);
-    b = block_best(b, sv, si);
+    const Cand b = row_best(x, begin < end ? begin : end, end, sv, si);
     if (threadIdx.x != 0 || b.i < 0) return;
     // Merge into the caller-initialised cell: replace the current holder when it is not a
     // valid index, holds a NaN, or loses under the ordering rule.

