@@ -137,6 +137,8 @@ def native():
     global _native
     if _native is None:
         lib()
+        import torch  # noqa: F401  (the module reads tensors through torch's own libraries, which must be loaded)
+
         try:
             from . import _native as module
         except ImportError as e:

@@ -123,8 +123,14 @@ def build_native(force=False):
     """The CPython module of the launch entry points, linked against the library beside it."""
     src = os.path.join(CSRC, "py_launch.cpp")
     if force or _newer(NATIVE, [src, os.path.join(os.path.dirname(HERE), "include", "rvllm_b200.h"), LIB]):
-        _run(["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], src, "-o", NATIVE,
-              "-L", HERE, "-l:librvllm_b200.so", "-Wl,-rpath,$ORIGIN"])
+        import torch
+        from torch.utils import cpp_extension
+
+        includes = [x for d in [sysconfig.get_paths()["include"], *cpp_extension.include_paths()] for x in ("-isystem", d)]
+        # (torch's libraries are in the process before the module is: no path to them is recorded)
+        _run(["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+              *includes, src, "-o", NATIVE, "-L", HERE, "-l:librvllm_b200.so", "-L", cpp_extension.library_paths()[0],
+              "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-Wl,-rpath,$ORIGIN"])
     return NATIVE
 
 

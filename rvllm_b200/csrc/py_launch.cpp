@@ -4,13 +4,16 @@
 // validates, stream look-up), several times the kernel at decode sizes; an executor that issues a layer call by call
 // is then bound by the interpreter (measured: 98 us for a layer of eight small kernels).  These wrappers are
 // METH_FASTCALL functions whose parameter types are deduced from the C prototypes, so a call costs its conversions only.
-// Pointers may be None, integers, or any object with a data_ptr() method (a tensor).  Every wrapper returns the C
-// function's status; reading the message and raising stays with the Python side.
+// Pointers may be None, integers, torch tensors (read in place: the data_ptr() method costs 0.15 us, and a layer passes 70
+// of them), or any other object with that method.  Every wrapper returns the C function's status; reading the message and
+// raising stays with the Python side.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 #include <stdint.h>
+#include <torch/csrc/autograd/python_variable.h>
 
+#include <exception>
 #include <tuple>
 #include <type_traits>
 #include <utility>
@@ -24,6 +27,15 @@ PyObject* g_data_ptr = nullptr;  // interned "data_ptr"
 bool to_pointer(PyObject* o, uintptr_t* out) {
     if (o == Py_None) {
         *out = 0;
+        return true;
+    }
+    if (THPVariable_Check(o)) {
+        try {
+            *out = reinterpret_cast<uintptr_t>(THPVariable_Unpack(o).data_ptr());
+        } catch (const std::exception& e) {
+            PyErr_SetString(PyExc_RuntimeError, e.what());
+            return false;
+        }
         return true;
     }
     if (PyLong_Check(o)) {
@@ -75,6 +87,79 @@ template <typename... A, int (*Fn)(A...)> struct Wrap<Fn> {
     }
 };
 
+// Calls that take their sizes from the tensors.  None instead of a status: an argument is not what this reads (the Python
+// side then goes the long way round, which raises what it always raised).
+const at::Tensor* as_tensor(PyObject* o, int64_t dims) {
+    if (!THPVariable_Check(o)) return nullptr;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    return t.dim() == dims ? &t : nullptr;
+}
+int kind_of(const at::Tensor& t) {
+    switch (t.scalar_type()) {
+        case at::kHalf: return RVLLM_OUT_F16;
+        case at::kBFloat16: return RVLLM_OUT_BF16;
+        case at::kFloat: return RVLLM_OUT_F32;
+        default: return -1;
+    }
+}
+bool fits_int(int64_t v) { return v >= 0 && v <= INT32_MAX; }
+
+// gemm(out, a_fp8, w_fp8, a_scale, w_scale, residual, impl, workspace, stream)
+PyObject* gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 9) return PyErr_Format(PyExc_TypeError, "expected 9 arguments, got %zd", n);
+    const at::Tensor *A = as_tensor(a[1], 2), *W = as_tensor(a[2], 2);
+    if (!A || !W || !THPVariable_Check(a[0])) Py_RETURN_NONE;
+    const int kind = kind_of(THPVariable_Unpack(a[0]));
+    const int64_t M = A->size(0), K = A->size(1), N = W->size(0);
+    if (kind < 0 || !fits_int(M) || !fits_int(N) || !fits_int(K)) Py_RETURN_NONE;
+    uintptr_t p[6], ws = 0, stream;
+    int impl;
+    size_t ws_len = 0;
+    for (int i = 0; i < 6; i++)
+        if (!to_pointer(a[i], &p[i])) return nullptr;
+    if (!convert(a[6], &impl) || !to_pointer(a[8], &stream)) return nullptr;
+    if (a[7] != Py_None) {
+        if (!THPVariable_Check(a[7])) Py_RETURN_NONE;
+        if (!to_pointer(a[7], &ws)) return nullptr;
+        ws_len = THPVariable_Unpack(a[7]).nbytes();
+    }
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = rvllm_fp8_gemm_channelscale((void*)p[0], kind, (const void*)p[1], (const void*)p[2], (const float*)p[3], (const float*)p[4],
+                                     (const void*)p[5], (int)M, (int)N, (int)K, impl, (void*)ws, ws_len, (void*)stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+}
+
+// rope(qkv, heads, kv_heads, head_dim, rotary_dim, cos, sin, positions, slots, q_fp8, q_scale, k_cache, v_cache, k_scale,
+//      v_scale, stream): the packed [T, (heads + 2 * kv_heads) * head_dim] row
+PyObject* rope(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 16) return PyErr_Format(PyExc_TypeError, "expected 16 arguments, got %zd", n);
+    const at::Tensor *x = as_tensor(a[0], 2), *cos = as_tensor(a[5], 2);
+    if (!x || !cos || !THPVariable_Check(a[13])) Py_RETURN_NONE;
+    const int dtype = kind_of(*x);
+    int heads, kv_heads, head_dim, rotary;
+    if (!convert(a[1], &heads) || !convert(a[2], &kv_heads) || !convert(a[3], &head_dim) || !convert(a[4], &rotary)) return nullptr;
+    const int64_t T = x->size(0), stride = x->size(1), positions = cos->size(0);
+    if ((dtype != RVLLM_F16 && dtype != RVLLM_BF16) || kv_heads <= 0 || !fits_int(T) || !fits_int(stride) || !fits_int(positions))
+        Py_RETURN_NONE;
+    const int64_t slots = THPVariable_Unpack(a[13]).numel() / kv_heads;
+    if (!fits_int(slots)) Py_RETURN_NONE;
+    uintptr_t base, p[10], stream;  // cos .. v_scale
+    if (!to_pointer(a[0], &base) || !to_pointer(a[15], &stream)) return nullptr;
+    for (int i = 0; i < 10; i++)
+        if (!to_pointer(a[5 + i], &p[i])) return nullptr;
+    const uintptr_t k_in = base + 2ull * heads * head_dim, v_in = k_in + 2ull * kv_heads * head_dim;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = rvllm_rope_fp8kv_launch((const void*)base, (const void*)k_in, (const void*)v_in, (int)stride, (void*)p[4], (void*)p[6],
+                                 (void*)p[7], (float*)p[8], (float*)p[9], (float*)p[5], (const void*)p[0], (const void*)p[1],
+                                 (const int32_t*)p[2], (const int32_t*)p[3], (int)T, heads, kv_heads, head_dim, rotary,
+                                 (int)positions, (int)slots, dtype, (void*)stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+}
+
 #define ENTRY(fn) {#fn, (PyCFunction)(void (*)(void))Wrap<fn>::call, METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {
     ENTRY(rvllm_fused_rmsnorm_fp8_quant_launch),
@@ -89,6 +174,8 @@ PyMethodDef g_methods[] = {
     ENTRY(rvllm_fp8_gemm_qkv_rope_fp8kv),
     ENTRY(rvllm_paged_decode_fp8),
     ENTRY(rvllm_paged_decode_fp8_quant),
+    {"gemm", (PyCFunction)(void (*)(void))gemm, METH_FASTCALL, nullptr},
+    {"rope", (PyCFunction)(void (*)(void))rope, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Launch entry points of librvllm_b200.so.", -1, g_methods,

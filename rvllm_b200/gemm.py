@@ -22,11 +22,18 @@ def _out_kind(t) -> int:
 def fp8_gemm_channelscale(out, a_fp8, w_fp8, a_scale, w_scale, residual=None, impl=IMPL_AUTO, workspace=None,
                           stream=None) -> None:
     """out[M, N] = cast(a_scale[m] * (w_scale[n] * A[M, K] . W[N, K]^T) (+ residual))."""
+    if stream is None:
+        stream = _lib.current_stream()
+    rc = native().gemm(out, a_fp8, w_fp8, a_scale, w_scale, residual, impl, workspace, stream)
+    if rc is not None:
+        if rc:
+            check(rc, "fp8_gemm_channelscale")
+        return
     M, K = a_fp8.shape
     N = w_fp8.shape[0]
     rc = native().rvllm_fp8_gemm_channelscale(out, _out_kind(out), a_fp8, w_fp8, a_scale, w_scale, residual, M, N, K, impl,
                                               workspace, 0 if workspace is None else workspace.nbytes,
-                                              _lib.current_stream() if stream is None else stream)
+                                              stream)
     if rc:
         check(rc, "fp8_gemm_channelscale")
 

@@ -143,6 +143,12 @@ class ArgmaxLaunch:
 def rope_fp8kv(qkv, heads, kv_heads, head_dim, rotary_dim, cos, sin, positions, slot_mapping, q_fp8, q_scale,
                k_cache, v_cache, k_scale_cache, v_scale_cache, stream=None) -> None:
     """RoPE + Q quantisation + paged FP8 KV write over a packed [T, (heads + 2*kv_heads)*head_dim] row."""
+    rc = native().rope(qkv, heads, kv_heads, head_dim, rotary_dim, cos, sin, positions, slot_mapping, q_fp8, q_scale, k_cache,
+                       v_cache, k_scale_cache, v_scale_cache, _stream(stream))
+    if rc is not None:
+        if rc:
+            check(rc, "rope_fp8kv")
+        return
     T, stride = qkv.shape
     es = qkv.element_size()
     q_dim, kv_dim = heads * head_dim, kv_heads * head_dim
@@ -160,6 +166,8 @@ def qkv_rope_fp8kv(a_fp8, w_fp8, a_scale, w_scale, heads, kv_heads, head_dim, co
                    q_scale, k_cache, v_cache, k_scale_cache, v_scale_cache, stream=None) -> bool:
     """QKV projection with RoPE + Q quantisation + paged FP8 KV write in the GEMM epilogue.  Returns
     False when the library does not take the shape (the caller then runs the GEMM and rope_fp8kv)."""
+    if head_dim != 128:
+        return False  # (one weight tile is one head: the library takes no other size)
     M, K = a_fp8.shape
     slots = k_scale_cache.numel() // kv_heads
     rc = native().rvllm_fp8_gemm_qkv_rope_fp8kv(a_fp8, w_fp8, a_scale, w_scale, M, K, heads, kv_heads, head_dim,

@@ -170,3 +170,22 @@ def test_library_is_not_the_time_stamp_build():
         assert L.rvllm_fp8_gemm_tc_trace(ctypes.c_void_p(4096), 1) == _lib.E_UNSUPPORTED
     finally:
         assert L.rvllm_fp8_gemm_tc_trace(None, 0) == _lib.OK
+
+
+def test_native_calls_that_read_tensors_refuse_what_they_cannot_read():
+    """The CPython module's tensor-sized calls answer None (the wrapper then goes through the plain entry point) for what is
+    no 2-D tensor of a known type, a status for what the library itself refuses."""
+    torch = pytest.importorskip("torch")
+    from rvllm_b200 import _lib
+    n = _lib.native()
+    x = torch.zeros((4, 64), dtype=torch.float16)
+    assert n.gemm(x, x, x, x, x, None, 9, None, 0) == _lib.E_INVALID          # impl out of range
+    assert n.gemm(x, x[0], x, x, x, None, 0, None, 0) is None
+    assert n.gemm(x.double(), x, x, x, x, None, 0, None, 0) is None
+    assert n.gemm(0, x, x, x, x, None, 0, None, 0) is None
+    assert n.rope(x[0], 1, 1, 64, 64, x, x, x, x, x, x, x, x, x, x, 0) is None
+    assert n.rope(x, 1, 1, 63, 0, x, x, x, x, x, x, x, x, x, x, 0) == _lib.E_INVALID
+    with pytest.raises(TypeError):
+        n.gemm(x)
+    with pytest.raises(AttributeError):
+        n.gemm(x, x, x, "scale", x, None, 0, None, 0)
