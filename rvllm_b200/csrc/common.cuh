@@ -120,7 +120,11 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // Per-row scale and its reciprocal: scale = max(absmax / 448, 1e-12).
 __device__ __forceinline__ float row_scale(float absmax) { return fmaxf(absmax / RV_FP8_MAX, 1e-12f); }
 
+// Weights and tables only (norm gains, RoPE and embedding tables: nothing in flight writes them).  A read-only load, like a
+// load through a __restrict__ argument, may be moved ahead of pdl_wait(), so it must not touch what a kernel of the chain
+// writes; those values are read with plain loads through pointers without __restrict__.
 __device__ __forceinline__ uint4 ldg128(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+__device__ __forceinline__ uint4 ld128(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 // Streaming 128-bit load that does not pollute L1 (weights and KV rows are read once).
 __device__ __forceinline__ uint4 ld_stream128(const void* p) {
     uint4 v;

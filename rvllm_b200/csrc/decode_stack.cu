@@ -39,49 +39,66 @@ __global__ void fill_tables_kernel(int* tables, int n, unsigned long long mul, u
 }
 
 // Per-step bookkeeping, on the device so that a graph replay needs no host input: slot of the token written at
-// position `pos`, for the global and the ring (sliding) layout, and the context length that includes it.
-__device__ __forceinline__ void place_token(int b, int pos, const int* __restrict__ tables_global,
-                                            const int* __restrict__ tables_sliding, int* __restrict__ slots_global,
-                                            int* __restrict__ slots_sliding, int* __restrict__ ctx_lens, int block_size,
-                                            int mb_global, int mb_sliding) {
+// position `pos`, for the global and the ring (sliding) layout, and the context length that includes it.  Looking up and
+// storing are apart: the compiler cannot move a load across a store through another of these pointers, and in the advance
+// kernel the look-ups are one dependent chain of a single block.
+struct Placed {
+    int slot_global, slot_sliding;
+};
+__device__ __forceinline__ Placed find_slots(int b, int pos, const int* tables_global, const int* tables_sliding, int block_size,
+                                             int mb_global, int mb_sliding) {
     const int page = pos / block_size, off = pos % block_size;
     const int blk = page < mb_global ? tables_global[b * mb_global + page] : -1;  // -1: no block dealt to this page
-    slots_global[b] = blk >= 0 ? blk * block_size + off : -1;
-    slots_sliding[b] = mb_sliding > 0 ? tables_sliding[b * mb_sliding + page % mb_sliding] * block_size + off : -1;
+    return {blk >= 0 ? blk * block_size + off : -1,
+            mb_sliding > 0 ? tables_sliding[b * mb_sliding + page % mb_sliding] * block_size + off : -1};
+}
+__device__ __forceinline__ void place_token(int b, int pos, Placed at, int* slots_global, int* slots_sliding, int* ctx_lens) {
+    slots_global[b] = at.slot_global;
+    slots_sliding[b] = at.slot_sliding;
     ctx_lens[b] = pos + 1;
 }
 // After a reset or a seeding: the bookkeeping of the first step.  Every later step finds what its predecessor's
 // advance_kernel left, so that inside a step nothing writes slots, context lengths or block tables: kernels of the step
 // may read them without waiting for the kernel before them.
-__global__ void prepare_step_kernel(const int* __restrict__ positions, const int* __restrict__ tables_global,
-                                    const int* __restrict__ tables_sliding, int* __restrict__ slots_global,
-                                    int* __restrict__ slots_sliding, int* __restrict__ ctx_lens, int batch,
+__global__ void prepare_step_kernel(const int* positions, const int* tables_global, const int* tables_sliding,
+                                    int* slots_global, int* slots_sliding, int* ctx_lens, int batch,
                                     int block_size, int mb_global, int mb_sliding) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= batch) return;
-    place_token(b, positions[b], tables_global, tables_sliding, slots_global, slots_sliding, ctx_lens, block_size, mb_global,
-                mb_sliding);
+    const int pos = positions[b];
+    place_token(b, pos, find_slots(b, pos, tables_global, tables_sliding, block_size, mb_global, mb_sliding), slots_global,
+                slots_sliding, ctx_lens);
 }
 
 // After argmax: record the emitted token, choose the next input token (prompt while it lasts,
 // then greedy feedback), advance the position and the step counter, and place the next step's token.  One block.
-__global__ void advance_kernel(int* __restrict__ tokens, const int* __restrict__ next, int* __restrict__ positions,
-                               const int* __restrict__ prompt, int prompt_len, int* __restrict__ history,
-                               int* __restrict__ step_counter, int max_steps, int batch,
-                               const int* __restrict__ tables_global, const int* __restrict__ tables_sliding,
-                               int* __restrict__ slots_global, int* __restrict__ slots_sliding, int* __restrict__ ctx_lens,
-                               int block_size, int mb_global, int mb_sliding) {
+// `early`: nothing in flight writes what it looks up besides the emitted tokens (a step of a graph starts behind a complete
+// predecessor), so the dependent chain step / position -> prompt token, table entries runs ahead of the wait for the merge.
+__global__ void advance_kernel(int* tokens, const int* next, int* positions, const int* prompt, int prompt_len, int* history,
+                               int* step_counter, int max_steps, int batch, const int* tables_global,
+                               const int* tables_sliding, int* slots_global, int* slots_sliding, int* ctx_lens,
+                               int block_size, int mb_global, int mb_sliding, int early) {
     rv::pdl_launch();
+    int step = 0, pos = 0, prompted = 0;
+    Placed at = {-1, -1};
+    auto look_up = [&](int b) {
+        pos = positions[b] + 1;
+        prompted = pos < prompt_len ? prompt[(size_t)b * prompt_len + pos] : 0;
+        at = find_slots(b, pos, tables_global, tables_sliding, block_size, mb_global, mb_sliding);
+    };
+    if (early) {
+        step = *step_counter;
+        if ((int)threadIdx.x < batch) look_up(threadIdx.x);
+    }
     rv::pdl_wait();
-    const int step = *step_counter;
+    if (!early) step = *step_counter;
     for (int b = threadIdx.x; b < batch; b += blockDim.x) {
-        const int pos = positions[b];
         const int emitted = next[b];
+        if (!early || b >= (int)blockDim.x) look_up(b);
         if (step < max_steps) history[(size_t)step * batch + b] = emitted;
-        tokens[b] = (pos + 1 < prompt_len) ? prompt[(size_t)b * prompt_len + pos + 1] : emitted;
-        positions[b] = pos + 1;
-        place_token(b, pos + 1, tables_global, tables_sliding, slots_global, slots_sliding, ctx_lens, block_size, mb_global,
-                    mb_sliding);
+        tokens[b] = pos < prompt_len ? prompted : emitted;
+        positions[b] = pos;
+        place_token(b, pos, at, slots_global, slots_sliding, ctx_lens);
     }
     __syncthreads();
     if (threadIdx.x == 0) *step_counter = step + 1;
@@ -479,7 +496,7 @@ int enqueue_step(rvllm_stack* s, int* launches, bool chained = false) {
     rv_launch(advance_kernel, dim3(1), dim3(256), 0, s->stream, dim3(1, 1, 1), s->tokens, s->next_tokens, s->positions, s->prompt, c.prompt_len,
                                              s->history, s->step_counter, c.max_steps, B, (const int*)s->tables_global,
                                              (const int*)s->tables_sliding, s->slots_global, s->slots_sliding, s->ctx_lens,
-                                             c.block_size, s->mb_global, s->mb_sliding);
+                                             c.block_size, s->mb_global, s->mb_sliding, s->capturing ? 1 : 0);
     RV_TRY(rv_launched("advance"));
     n += 1;
     if (launches) *launches = n;

@@ -35,14 +35,14 @@ __device__ __forceinline__ bool good_scale(float s) { return isfinite(s) && s > 
 }  // namespace
 
 extern "C" __global__ void __launch_bounds__(FA2_THREADS)
-flash_attention_2_decode_fp8kv_kernel(__half* __restrict__ output, const unsigned char* __restrict__ query,
-                                      const unsigned char* __restrict__ key_cache,
-                                      const unsigned char* __restrict__ value_cache,
-                                      const float* __restrict__ k_scale_cache, const float* __restrict__ v_scale_cache,
-                                      const float* __restrict__ q_scale_cache,
-                                      const float* __restrict__ k_descale_fallback,
-                                      const float* __restrict__ v_descale_fallback, const int* __restrict__ block_tables,
-                                      const int* __restrict__ context_lens, const float* __restrict__ q_descale,
+flash_attention_2_decode_fp8kv_kernel(__half* __restrict__ output, const unsigned char* query,
+                                      const unsigned char* key_cache,
+                                      const unsigned char* value_cache,
+                                      const float* k_scale_cache, const float* v_scale_cache,
+                                      const float* q_scale_cache,
+                                      const float* k_descale_fallback,
+                                      const float* v_descale_fallback, const int* block_tables,
+                                      const int* context_lens, const float* q_descale,
                                       float scale, int num_heads, int num_kv_heads, int head_dim, int block_size,
                                       int max_blocks_per_seq, int window_size_left, int num_blocks_total) {
     __shared__ int invalid_table;
@@ -75,9 +75,9 @@ flash_attention_2_decode_fp8kv_kernel(__half* __restrict__ output, const unsigne
     if (invalid_table) return;
 
     const int kvh = num_kv_heads == num_heads ? head : head / (num_heads / num_kv_heads);
-    const float q_scale = q_scale_cache ? __ldg(q_scale_cache + (long long)seq * num_heads + head) : *q_descale;
-    const float k_scalar = k_perslot ? 0.0f : __ldg(k_descale_fallback);
-    const float v_scalar = v_perslot ? 0.0f : __ldg(v_descale_fallback);
+    const float q_scale = q_scale_cache ? q_scale_cache[(long long)seq * num_heads + head] : *q_descale;
+    const float k_scalar = k_perslot ? 0.0f : *k_descale_fallback;
+    const float v_scalar = v_perslot ? 0.0f : *v_descale_fallback;
     if (!good_scale(q_scale) || (!k_perslot && !good_scale(k_scalar)) || (!v_perslot && !good_scale(v_scalar))) return;
     const int start = window_size_left < 0 ? 0 : max(0, ctx - 1 - window_size_left);
 
@@ -116,8 +116,8 @@ flash_attention_2_decode_fp8kv_kernel(__half* __restrict__ output, const unsigne
         const int page = pos / block_size;
         const long long slot = (long long)table[page] * block_size + (pos - page * block_size);
         const long long row = slot * num_kv_heads + kvh;
-        const float ks = k_perslot ? __ldg(k_scale_cache + row) : k_scalar;
-        const float vs = v_perslot ? __ldg(v_scale_cache + row) : v_scalar;
+        const float ks = k_perslot ? k_scale_cache[row] : k_scalar;
+        const float vs = v_perslot ? v_scale_cache[row] : v_scalar;
         if (!good_scale(ks) || !good_scale(vs)) poisoned = true;
         float dot = 0.0f;
         float vf[MAX_PIECES][8];
@@ -127,8 +127,8 @@ flash_attention_2_decode_fp8kv_kernel(__half* __restrict__ output, const unsigne
 #pragma unroll
             for (int j = 0; j < 8; j++) vf[pc][j] = 0.0f;
             if (pc < pieces && d0 < head_dim) {
-                const uint2 kr = __ldg(reinterpret_cast<const uint2*>(key_cache + row * head_dim + d0));
-                const uint2 vr = __ldg(reinterpret_cast<const uint2*>(value_cache + row * head_dim + d0));
+                const uint2 kr = *reinterpret_cast<const uint2*>(key_cache + row * head_dim + d0);
+                const uint2 vr = *reinterpret_cast<const uint2*>(value_cache + row * head_dim + d0);
                 float kf[8];
                 rv::e4m3x4_to_f32x4(kr.x, kf);
                 rv::e4m3x4_to_f32x4(kr.y, kf + 4);

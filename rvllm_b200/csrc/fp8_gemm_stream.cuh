@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(THREADS, (NT8 <= 4 ? 2 : 1)) fp8_gemm_stream_k
         for (int u = 0; u < 2; u++) {
 #pragma unroll
             for (int i = 0; i < NT8; i++) {
-                const uint4 av = rv::ldg128(arow[i] + (size_t)(c + u) * CHUNK);
+                const uint4 av = rv::ld128(arow[i] + (size_t)(c + u) * CHUNK);
                 mma_e4m3(acc[0][i], wv[u][0].x, wv[u][1].x, wv[u][0].y, wv[u][1].y, av.x, av.y);
                 mma_e4m3(acc[0][i], wv[u][0].z, wv[u][1].z, wv[u][0].w, wv[u][1].w, av.z, av.w);
                 mma_e4m3(acc[1][i], wv[u][2].x, wv[u][3].x, wv[u][2].y, wv[u][3].y, av.x, av.y);
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(THREADS, (NT8 <= 4 ? 2 : 1)) fp8_gemm_stream_k
         for (int r = 0; r < 4; r++) wv[r] = rv::ld_stream128(wrow[r] + (size_t)c * CHUNK);
 #pragma unroll
         for (int i = 0; i < NT8; i++) {
-            const uint4 av = rv::ldg128(arow[i] + (size_t)c * CHUNK);
+            const uint4 av = rv::ld128(arow[i] + (size_t)c * CHUNK);
             mma_e4m3(acc[0][i], wv[0].x, wv[1].x, wv[0].y, wv[1].y, av.x, av.y);
             mma_e4m3(acc[0][i], wv[0].z, wv[1].z, wv[0].w, wv[1].w, av.z, av.w);
             mma_e4m3(acc[1][i], wv[2].x, wv[3].x, wv[2].y, wv[3].y, av.x, av.y);

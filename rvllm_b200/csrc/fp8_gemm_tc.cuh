@@ -336,8 +336,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 nx[q][0] = nx[q][1] = make_uint4(0, 0, 0, 0);
                 if (c < BN * 8 && i < nkb && m < p.M && k0 < p.K) {
                     const uint4* src = reinterpret_cast<const uint4*>(a16 + (size_t)m * p.K + k0);
-                    nx[q][0] = rv::ldg128(src);
-                    nx[q][1] = rv::ldg128(src + 1);
+                    nx[q][0] = rv::ld128(src);
+                    nx[q][1] = rv::ld128(src + 1);
                 }
             }
         }
@@ -885,7 +885,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 }
 
 // Second half of the fused greedy tail: the row's winner over the per-tile winners.  grid = rows, block = 256.
-__global__ void __launch_bounds__(256) argmax_merge_kernel(const float* __restrict__ val, const int* __restrict__ idx,
+__global__ void __launch_bounds__(256) argmax_merge_kernel(const float* val, const int* idx,
                                                           int tiles, int* __restrict__ out) {
     __shared__ float sv[8];
     __shared__ int si[8];

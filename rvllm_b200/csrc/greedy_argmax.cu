@@ -167,7 +167,7 @@ extern "C" __global__ void argmax_kernel(const float* logits, int* __restrict__ 
     if (threadIdx.x == 0) out[row] = b.i;
 }
 
-extern "C" __global__ void argmax_f16_kernel(const __half* __restrict__ logits, int* __restrict__ out, int vocab) {
+extern "C" __global__ void argmax_f16_kernel(const __half* logits, int* __restrict__ out, int vocab) {
     __shared__ float sv[32];
     __shared__ int si[32];
     rv::pdl_launch();

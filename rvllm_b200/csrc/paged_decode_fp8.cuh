@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(THREADS) paged_decode_fp8_kernel(Params p) {
     if (tbl_in_smem)
         for (int i = tid; i <= last_page - first_page; i += THREADS) {
             const int page = first_page + i;
-            tbl[i] = __ldg(table + (p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page));
+            tbl[i] = table[p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page];
         }
     __syncthreads();
 
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(THREADS) paged_decode_fp8_kernel(Params p) {
             const int head = kvh * group + h0 + (j < nh ? j : 0);
             const float q_ds = p.q_scale_cache ? p.q_scale_cache[(size_t)b * p.heads + head] : *p.q_descale;
             if (bad_scale(q_ds)) bad |= 1u << j;
-            const uint4 qv = rv::ldg128(p.q + ((size_t)b * p.heads + head) * HD + 16 * sub);
+            const uint4 qv = rv::ld128(p.q + ((size_t)b * p.heads + head) * HD + 16 * sub);
             dequant16(qv, q[j]);
 #pragma unroll
             for (int d = 0; d < 16; d++) q[j][d] *= q_ds;
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(THREADS) paged_decode_fp8_kernel(Params p) {
                     phys = tbl[page - first_page];
                 } else {
                     const int tpage = p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page;
-                    phys = __ldg(table + tpage);
+                    phys = table[tpage];
                 }
                 if (phys < 0 || phys >= p.num_blocks_total) {
                     bad = 0xffffffffu;
@@ -350,8 +350,8 @@ __global__ void __launch_bounds__(THREADS) paged_decode_fp8_kernel(Params p) {
 
 // grid = (batch * heads), block = min(HD, 256): LSE merge of a sequence's chunks.
 template <int HD, typename OutT>
-__global__ void paged_decode_fp8_combine_kernel(const float* __restrict__ workspace, OutT* __restrict__ out,
-                                                const int* __restrict__ context_lens, int heads, int block_size,
+__global__ void paged_decode_fp8_combine_kernel(const float* workspace, OutT* __restrict__ out,
+                                                const int* context_lens, int heads, int block_size,
                                                 int max_blocks_per_seq, int window_size_left, int max_chunks,
                                                 int min_chunk_tokens) {
     constexpr int PSTRIDE = HD + 2;
@@ -388,8 +388,8 @@ __global__ void paged_decode_fp8_combine_kernel(const float* __restrict__ worksp
 // force_partial, so every (head, chunk) partial is in the workspace.
 template <int HD, typename OutT>
 __global__ void __launch_bounds__(512)
-paged_decode_fp8_combine_quant_kernel(const float* __restrict__ workspace, uint8_t* __restrict__ out_fp8,
-                                      float* __restrict__ out_scale, const int* __restrict__ context_lens, int heads,
+paged_decode_fp8_combine_quant_kernel(const float* workspace, uint8_t* __restrict__ out_fp8,
+                                      float* __restrict__ out_scale, const int* context_lens, int heads,
                                       int block_size, int max_blocks_per_seq, int window_size_left, int max_chunks,
                                       int min_chunk_tokens) {
     constexpr int PSTRIDE = HD + 2;

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(MMA_THREADS, (GT <= 2 ? 4 : 3)) paged_decode_f
     if (tbl_in_smem)
         for (int i = tid; i <= last_page - first_page; i += MMA_THREADS) {
             const int page = first_page + i;
-            tbl[i] = __ldg(table + (p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page));
+            tbl[i] = table[p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page];
         }
     __syncthreads();
 
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(MMA_THREADS, (GT <= 2 ? 4 : 3)) paged_decode_f
         if (tbl_in_smem) {
             phys = tbl[page - first_page];
         } else {
-            phys = __ldg(table + (p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page));
+            phys = table[p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page];
         }
         if (phys < 0 || phys >= p.num_blocks_total) {
             bad = 0xffffffffu;
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(MMA_THREADS, (GT <= 2 ? 4 : 3)) paged_decode_f
             const uint8_t* qrow = p.q + ((size_t)b * p.heads + head) * HD;
 #pragma unroll
             for (int c = 0; c < CH; c++)
-                qf[c] = g < nh ? rv::ldg128(qrow + c * 64 + 16 * t) : make_uint4(0, 0, 0, 0);
+                qf[c] = g < nh ? rv::ld128(qrow + c * 64 + 16 * t) : make_uint4(0, 0, 0, 0);
         }
         // this lane's score columns are heads 2t and 2t+1 of the tile: q scale * softmax scale
         float qsc[2];

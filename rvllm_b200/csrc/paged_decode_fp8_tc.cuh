@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(MMA_THREADS, (HD <= 128 ? 4 : 3)) paged_decode
     if (tbl_in_smem)
         for (int i = tid; i <= last_page - first_page; i += MMA_THREADS) {
             const int page = first_page + i;
-            tbl[i] = __ldg(table + (p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page));
+            tbl[i] = table[p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page];
         }
     __syncthreads();
 
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(MMA_THREADS, (HD <= 128 ? 4 : 3)) paged_decode
         if (tbl_in_smem) {
             phys = tbl[page - first_page];
         } else {
-            phys = __ldg(table + (p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page));
+            phys = table[p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page];
         }
         if ((unsigned)phys >= (unsigned)p.num_blocks_total) {
             bad = 0xffffffffu;
@@ -214,13 +214,13 @@ __global__ void __launch_bounds__(MMA_THREADS, (HD <= 128 ? 4 : 3)) paged_decode
                 if (warp == 0) {
 #pragma unroll
                     for (int c = 0; c < CH; c++)
-                        q_sm[c * 32 + lane] = g < nh ? rv::ldg128(qrow + c * 64 + 16 * t) : make_uint4(0, 0, 0, 0);
+                        q_sm[c * 32 + lane] = g < nh ? rv::ld128(qrow + c * 64 + 16 * t) : make_uint4(0, 0, 0, 0);
                 }
                 __syncthreads();
             } else {
 #pragma unroll
                 for (int c = 0; c < CH; c++)
-                    qf[c] = g < nh ? rv::ldg128(qrow + c * 64 + 16 * t) : make_uint4(0, 0, 0, 0);
+                    qf[c] = g < nh ? rv::ld128(qrow + c * 64 + 16 * t) : make_uint4(0, 0, 0, 0);
             }
         }
         // this lane's score columns are heads 2t and 2t+1 of the tile: q scale * softmax scale * log2(e)

@@ -304,32 +304,40 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
     // "this CTA runs and its barriers exist": the other CTAs of the cluster wait for this before they touch its memory
     if constexpr (CL) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     const uint32_t tmem_base = *tmem_holder;
-    const int nh = group < GT ? group : GT;  // query heads of this KV head (the launcher guarantees group <= GT)
-    if (warp != 0) {
-        // The producer warp goes straight to its loads; the other five warps stage Q meanwhile.
-        if (early) rv::pdl_wait();  // Q, and the newest token's scales, come from the preceding kernel
-        if (active) {
-            // Q codes of the KV head's query heads -> B operand panels (K-major, swizzled by hand)
-            for (int i = tid - 32; i < nh * (HD / 16); i += THREADS - 32) {
-                const int n = i / (HD / 16), c = i % (HD / 16), h = c >> 3, cc = c & 7;
-                const uint4 v = rv::ldg128(p.q + ((size_t)b * p.heads + (size_t)kvh * group + n) * HD + c * 16);
-                *reinterpret_cast<uint4*>(q_tile + h * (NQ * PANEL) + n * PANEL + ((cc ^ (n & 7)) << 4)) = v;
-            }
-        }
-        fence_proxy_async();  // P / Q tiles were written through the generic proxy; the MMAs read them through the async one
-        asm volatile("bar.sync 2, 160;" ::: "memory");
-    }
-
     // physical block of the page holding `tok` (integer divisions only off the common power-of-two path)
-    auto phys_of = [&](int tok, bool& bad_page) -> int {
+    auto block_of = [&](int tok) -> int {
         const int page = p.bs_shift >= 0 ? (tok >> p.bs_shift) : tok / bs;
-        const int ph = __ldg(table + (p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page));
+        return table[p.window_size_left >= 0 ? page % p.max_blocks_per_seq : page];
+    };
+    auto phys_of = [&](int tok, bool& bad_page) -> int {
+        const int ph = block_of(tok);
         if ((unsigned)ph >= (unsigned)p.num_blocks_total) {
             bad_page = true;
             return 0;
         }
         return ph;
     };
+
+    const int nh = group < GT ? group : GT;  // query heads of this KV head (the launcher guarantees group <= GT)
+    int ph_first = 0;
+    if (warp != 0) {
+        // The producer warp goes straight to its loads; the other five warps stage Q meanwhile.
+        if (early) rv::pdl_wait();  // Q, and the newest token's scales, come from the preceding kernel
+        if (active) {
+            if (warp >= 2) {  // softmax warps: the block of this thread's first token, on its way while Q is staged
+                const int tok = tile0 + ((warp & 3) * 32 + lane);
+                if (tok >= t_begin && tok < t_end) ph_first = block_of(tok);
+            }
+            // Q codes of the KV head's query heads -> B operand panels (K-major, swizzled by hand)
+            for (int i = tid - 32; i < nh * (HD / 16); i += THREADS - 32) {
+                const int n = i / (HD / 16), c = i % (HD / 16), h = c >> 3, cc = c & 7;
+                const uint4 v = rv::ld128(p.q + ((size_t)b * p.heads + (size_t)kvh * group + n) * HD + c * 16);
+                *reinterpret_cast<uint4*>(q_tile + h * (NQ * PANEL) + n * PANEL + ((cc ^ (n & 7)) << 4)) = v;
+            }
+        }
+        fence_proxy_async();  // P / Q tiles were written through the generic proxy; the MMAs read them through the async one
+        asm volatile("bar.sync 2, 160;" ::: "memory");
+    }
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer (whole warp)
@@ -501,19 +509,22 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
             m_run[k] = -1e20f;
             l_part[k] = 0.0f;
         }
-        // this thread's token of a tile: validity and its K / V scales (fetched one tile ahead)
+        // this thread's token of a tile: validity and its K / V scales (fetched one tile ahead; the first tile's table entry
+        // comes from before the barrier)
         auto fetch = [&](int i, bool& valid, float& ks, float& vs) {
             const int tok = tile0 + i * TOK + row;
             valid = i < ntiles && tok >= t_begin && tok < t_end;
             ks = k_scalar;
             vs = v_scalar;
             if (valid) {
-                bool bad_page = false;
-                const int ph = phys_of(tok, bad_page);
-                if (bad_page) bad = 0xffffffffu;  // a table entry outside the cache poisons the whole row
+                int ph = i == 0 ? ph_first : block_of(tok);
+                if ((unsigned)ph >= (unsigned)p.num_blocks_total) {
+                    bad = 0xffffffffu;  // a table entry outside the cache poisons the whole row
+                    ph = 0;
+                }
                 const size_t sidx = ((size_t)ph * bs + (tok % bs)) * p.kv_heads + kvh;
-                if (k_perslot) ks = __ldg(p.k_scale_cache + sidx);
-                if (v_perslot) vs = __ldg(p.v_scale_cache + sidx);
+                if (k_perslot) ks = p.k_scale_cache[sidx];
+                if (v_perslot) vs = p.v_scale_cache[sidx];
             }
         };
         bool valid_n, alive = true;

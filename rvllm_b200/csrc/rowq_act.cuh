@@ -40,7 +40,7 @@ __device__ __forceinline__ void mul8(const uint4& gv, const uint4& uv, float* y)
 
 template <int ACT, typename T>
 __device__ __forceinline__ void act_mul_quant_row(uint8_t* __restrict__ out, float* __restrict__ scales,
-                                                  const T* __restrict__ gate_up, int inter) {
+                                                  const T* gate_up, int inter) {
     constexpr int CACHE_VECS = 4;
     __shared__ float red[33];
     __shared__ int bad;
@@ -63,8 +63,8 @@ __device__ __forceinline__ void act_mul_quant_row(uint8_t* __restrict__ out, flo
     int c = 0;
     for (int v = tid; v < nvec; v += nt, c++) {
         float y[8];
-        mul8<ACT, T>(rv::ldg128(reinterpret_cast<const uint4*>(g) + v),
-                     rv::ldg128(reinterpret_cast<const uint4*>(u) + v), y);
+        mul8<ACT, T>(rv::ld128(reinterpret_cast<const uint4*>(g) + v),
+                     rv::ld128(reinterpret_cast<const uint4*>(u) + v), y);
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             nonfinite |= !isfinite(y[j]);
@@ -95,8 +95,8 @@ __device__ __forceinline__ void act_mul_quant_row(uint8_t* __restrict__ out, flo
                     for (int j = 0; j < 8; j++) y[j] = cache[k * 8 + j];
                 }
         } else {
-            mul8<ACT, T>(rv::ldg128(reinterpret_cast<const uint4*>(g) + v),
-                         rv::ldg128(reinterpret_cast<const uint4*>(u) + v), y);
+            mul8<ACT, T>(rv::ld128(reinterpret_cast<const uint4*>(g) + v),
+                         rv::ld128(reinterpret_cast<const uint4*>(u) + v), y);
         }
         uint2 w;
         w.x = rv::f32x4_to_e4m3x4(y[0] * inv, y[1] * inv, y[2] * inv, y[3] * inv);
@@ -119,7 +119,7 @@ constexpr int CLUSTER_THREADS = 256;
 // grid run as one wave -- the kernel is one latency chain per CTA, so a second wave doubles its time.
 template <int ACT, typename T, int CLUSTER_CACHE_VECS, int MINB>
 __global__ void __launch_bounds__(CLUSTER_THREADS, MINB)
-act_mul_quant_cluster_kernel(uint8_t* __restrict__ out, float* __restrict__ scales, const T* __restrict__ gate_up, int inter) {
+act_mul_quant_cluster_kernel(uint8_t* __restrict__ out, float* __restrict__ scales, const T* gate_up, int inter) {
     namespace cg = cooperative_groups;
     __shared__ float red[33];
     __shared__ int bad;
@@ -143,8 +143,8 @@ act_mul_quant_cluster_kernel(uint8_t* __restrict__ out, float* __restrict__ scal
     int c = 0;
     for (int v = v_lo + tid; v < v_hi; v += CLUSTER_THREADS, c++) {
         float y[8];
-        mul8<ACT, T>(rv::ldg128(reinterpret_cast<const uint4*>(g) + v),
-                     rv::ldg128(reinterpret_cast<const uint4*>(u) + v), y);
+        mul8<ACT, T>(rv::ld128(reinterpret_cast<const uint4*>(g) + v),
+                     rv::ld128(reinterpret_cast<const uint4*>(u) + v), y);
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             nonfinite |= !isfinite(y[j]);
@@ -189,8 +189,8 @@ act_mul_quant_cluster_kernel(uint8_t* __restrict__ out, float* __restrict__ scal
                     for (int j = 0; j < 8; j++) y[j] = cache[k * 8 + j];
                 }
         } else {
-            mul8<ACT, T>(rv::ldg128(reinterpret_cast<const uint4*>(g) + v),
-                         rv::ldg128(reinterpret_cast<const uint4*>(u) + v), y);
+            mul8<ACT, T>(rv::ld128(reinterpret_cast<const uint4*>(g) + v),
+                         rv::ld128(reinterpret_cast<const uint4*>(u) + v), y);
         }
         uint2 w;
         w.x = rv::f32x4_to_e4m3x4(y[0] * inv, y[1] * inv, y[2] * inv, y[3] * inv);

@@ -31,7 +31,7 @@ __device__ __forceinline__ float dec1(unsigned char v) {
 
 template <typename T>
 __device__ __forceinline__ void gemv_blockscale_body(T* __restrict__ output, const unsigned char* __restrict__ weight,
-                                                     const float* __restrict__ scale, const T* __restrict__ input, int M,
+                                                     const float* __restrict__ scale, const T* input, int M,
                                                      int N, int K, int num_col_blocks) {
     rv::pdl_launch();
     rv::pdl_wait();
@@ -62,8 +62,8 @@ __device__ __forceinline__ void gemv_blockscale_body(T* __restrict__ output, con
     };
     const bool vec_x = (reinterpret_cast<uintptr_t>(x_row) & 15) == 0 && (K & 7) == 0;
     auto load_x = [&](int k) -> uint4 {
-        if (vec_x) return rv::ldg128(x_row + k);
-        const uint2 lo = __ldg(reinterpret_cast<const uint2*>(x_row + k)), hi = __ldg(reinterpret_cast<const uint2*>(x_row + k + 4));
+        if (vec_x) return rv::ld128(x_row + k);
+        const uint2 lo = *reinterpret_cast<const uint2*>(x_row + k), hi = *reinterpret_cast<const uint2*>(x_row + k + 4);
         return make_uint4(lo.x, lo.y, hi.x, hi.y);
     };
     int k = lane * 8;

@@ -22,8 +22,8 @@ constexpr int STAGE_ELEMS = 16384;  // 32 KB of 16-bit values; longer rows strea
 
 template <typename T>
 __device__ __forceinline__ void rmsnorm_quant_row(uint8_t* __restrict__ out, float* __restrict__ scales,
-                                                  T* __restrict__ residual_out, const T* __restrict__ in,
-                                                  const T* __restrict__ residual, const T* __restrict__ gamma,
+                                                  T* residual_out, const T* in,
+                                                  const T* residual, const T* __restrict__ gamma,
                                                   float eps, int hidden) {
     __shared__ __align__(16) T srow[STAGE_ELEMS];
     rv::pdl_launch();
@@ -48,18 +48,35 @@ __device__ __forceinline__ void rmsnorm_quant_row(uint8_t* __restrict__ out, flo
     if (residual != nullptr) {
         // sum of squares of the unrounded sum, in thread-strided order; the rounded sum is
         // what the later passes normalise (reference :129-131,143).
+        // Four elements are read before the first of them is stored: residual_out may be residual (or in) itself, so the
+        // compiler cannot move a read across a store.
         const T* r = residual + base;
-        for (int i = tid; i < hidden; i += nt) {
-            float v = rv::T16<T>::to_f32(x[i]) + rv::T16<T>::to_f32(r[i]);
-            T h = rv::T16<T>::from_f32(v);
-            residual_out[base + i] = h;
-            if (staged) srow[i] = h;
-            ss += v * v;
+        constexpr int AHEAD = 4;
+        for (int i0 = tid; i0 < hidden; i0 += AHEAD * nt) {
+            T xa[AHEAD], ra[AHEAD];
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++) {
+                const int i = i0 + u * nt;
+                if (i < hidden) {
+                    xa[u] = x[i];
+                    ra[u] = r[i];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++) {
+                const int i = i0 + u * nt;
+                if (i >= hidden) break;
+                float v = rv::T16<T>::to_f32(xa[u]) + rv::T16<T>::to_f32(ra[u]);
+                T h = rv::T16<T>::from_f32(v);
+                residual_out[base + i] = h;
+                if (staged) srow[i] = h;
+                ss += v * v;
+            }
         }
     } else if (staged) {
         const int nvec = hidden >> 3;
         for (int v = tid; v < nvec; v += nt)
-            reinterpret_cast<uint4*>(srow)[v] = rv::ldg128(reinterpret_cast<const uint4*>(x) + v);
+            reinterpret_cast<uint4*>(srow)[v] = rv::ld128(reinterpret_cast<const uint4*>(x) + v);
         __syncthreads();
         for (int i = tid; i < hidden; i += nt) {
             float v = rv::T16<T>::to_f32(srow[i]);
@@ -152,7 +169,7 @@ __device__ __forceinline__ void rmsnorm_quant_row(uint8_t* __restrict__ out, flo
 
 template <typename T>
 __device__ __forceinline__ void quant_row(uint8_t* __restrict__ out, float* __restrict__ scales,
-                                          const T* __restrict__ in, int dim) {
+                                          const T* in, int dim) {
     __shared__ float red[33];
     rv::pdl_launch();
     rv::pdl_wait();
@@ -168,7 +185,7 @@ __device__ __forceinline__ void quant_row(uint8_t* __restrict__ out, float* __re
     float amax = 0.0f;
     if (vec_ok) {
         for (int v = tid; v < nvec; v += nt) {
-            uint4 xv = rv::ldg128(reinterpret_cast<const uint4*>(x) + v);
+            uint4 xv = rv::ld128(reinterpret_cast<const uint4*>(x) + v);
             if (v == tid) keep = xv;
             const uint32_t* xp = &xv.x;
 #pragma unroll
@@ -186,7 +203,7 @@ __device__ __forceinline__ void quant_row(uint8_t* __restrict__ out, float* __re
     const float inv = 1.0f / scale;
     if (vec_ok) {
         for (int v = tid; v < nvec; v += nt) {
-            uint4 xv = (v == tid) ? keep : rv::ldg128(reinterpret_cast<const uint4*>(x) + v);
+            uint4 xv = (v == tid) ? keep : rv::ld128(reinterpret_cast<const uint4*>(x) + v);
             const uint32_t* xp = &xv.x;
             float f[8];
 #pragma unroll

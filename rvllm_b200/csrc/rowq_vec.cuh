@@ -7,8 +7,7 @@
 // add + norm + quant 17.6 -> 7.0, RoPE + KV write 33.9 -> 10.7, act + quant 47.3 -> 28.4, per-token quant (4096) 8.0 -> 3.1;
 // on 32 rows the norm 4.1 -> 2.9.
 //
-// (What a preceding kernel wrote is read through plain pointers: a kernel argument that is const and __restrict__ may be
-// loaded ahead of the wait for that kernel.)
+// (What a preceding kernel wrote is read with plain loads: see rv::ldg128.)
 #pragma once
 #include "common.cuh"
 #include "rowq_act.cuh"
@@ -172,7 +171,7 @@ constexpr uint32_t ROW_WAIT_LIMIT = 1u << 24;
 
 template <int ACT, typename T, int NC>
 __global__ void __launch_bounds__(1024, 1) act_mul_quant_stream_kernel(uint8_t* __restrict__ out, float* __restrict__ scales,
-                                                                       const T* __restrict__ gate_up, int inter, int rows) {
+                                                                       const T* gate_up, int inter, int rows) {
     extern __shared__ __align__(128) uint8_t raw[];
     __shared__ uint64_t full[2];
     __shared__ uint32_t red[2][32];
