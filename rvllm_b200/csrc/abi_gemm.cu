@@ -237,6 +237,7 @@ int rvllm_fp8_gemm_qkv_rope_fp8kv(const void* a_fp8, const void* w_fp8, const fl
         !v_scale_cache || !cos_table || !sin_table || !positions || !slot_mapping)
         return rv_fail(RVLLM_E_INVALID, "null device pointer");
     if (!rv_aligned(a_fp8, 16) || !rv_aligned(w_fp8, 16)) return rv_fail(RVLLM_E_INVALID, "a / w must be 16-byte aligned");
+    if (!rv_aligned(cos_table, 2) || !rv_aligned(sin_table, 2)) return rv_fail(RVLLM_E_INVALID, "tables must be 2-byte aligned");
     rvtc::TcArgs t = {};
     t.out = nullptr;
     t.out_kind = dtype;
@@ -251,9 +252,6 @@ int rvllm_fp8_gemm_qkv_rope_fp8kv(const void* a_fp8, const void* w_fp8, const fl
     rvtc::RopeKv rk = {(uint8_t*)q_fp8, q_scale, (uint8_t*)k_cache, (uint8_t*)v_cache, k_scale_cache, v_scale_cache,
                        cos_table, sin_table, positions, slot_mapping, heads, kv_heads, max_positions, num_cache_slots};
     const int dt = dtype == RVLLM_F16 ? 0 : 1;
-    if (M > 32 && (!rv_aligned(cos_table, 4) || !rv_aligned(sin_table, 4) || !rv_aligned(q_fp8, 2) || !rv_aligned(k_cache, 2) ||
-                   !rv_aligned(v_cache, 2)))
-        return rv_fail(RVLLM_E_UNSUPPORTED, "fused QKV epilogue: tables must be 4-byte, Q and caches 2-byte aligned above 32 rows");
     const int rc = M > 32 ? rvpair::launch_pair_qkv_rope(t, rk, dt, (cudaStream_t)stream)
                           : rvtc::launch_qkv_rope(t, rk, dt, (cudaStream_t)stream);
     if (rc == -3) return RVLLM_E_UNSUPPORTED;  // message already recorded

@@ -52,6 +52,7 @@ struct PairParams {
     int stages, splits;
     int ranges, npart, sets;  // K ranges (V), most of them in one pair, sets of npart accumulators in tensor memory
     RopeKv rope;     // EPI_QKV_ROPE only
+    int rope_pairs;  // EPI_QKV_ROPE: tables 4-byte, Q and caches 2-byte aligned (a lane's two elements move as one)
     float* arg_val;  // EPI_ARGMAX only: as in TcParams
     int* arg_idx;
     float softcap;
@@ -304,8 +305,16 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 pos[i] = s_pos[b * 256 + g * 16 + quarter * 4 + i];
                 cw[i] = sw[i] = 0u;
                 if (kind != 2 && pos[i] >= 0 && pos[i] < rk.max_positions) {
-                    cw[i] = __ldg(reinterpret_cast<const uint32_t*>(rk.cos_t) + (size_t)pos[i] * 32 + lane);
-                    sw[i] = __ldg(reinterpret_cast<const uint32_t*>(rk.sin_t) + (size_t)pos[i] * 32 + lane);
+                    const size_t e = (size_t)pos[i] * 32 + lane;  // this lane's pair of table elements
+                    if (p.rope_pairs) {
+                        cw[i] = __ldg(reinterpret_cast<const uint32_t*>(rk.cos_t) + e);
+                        sw[i] = __ldg(reinterpret_cast<const uint32_t*>(rk.sin_t) + e);
+                    } else {
+                        const unsigned short *ct = reinterpret_cast<const unsigned short*>(rk.cos_t) + 2 * e,
+                                             *st = reinterpret_cast<const unsigned short*>(rk.sin_t) + 2 * e;
+                        cw[i] = (uint32_t)ct[0] | (uint32_t)ct[1] << 16;
+                        sw[i] = (uint32_t)st[0] | (uint32_t)st[1] << 16;
+                    }
                 }
             }
 #pragma unroll
@@ -346,8 +355,15 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     o = (kind == 1 ? rk.k_cache : rk.v_cache) + sidx * TILE_W;
                     so = (kind == 1 ? rk.k_scale : rk.v_scale) + sidx;
                 }
-                reinterpret_cast<unsigned short*>(o)[lane] = (unsigned short)(q & 0xffffu);
-                reinterpret_cast<unsigned short*>(o)[32 + lane] = (unsigned short)(q >> 16);
+                if (p.rope_pairs) {
+                    reinterpret_cast<unsigned short*>(o)[lane] = (unsigned short)(q & 0xffffu);
+                    reinterpret_cast<unsigned short*>(o)[32 + lane] = (unsigned short)(q >> 16);
+                } else {
+                    o[2 * lane] = (uint8_t)q;
+                    o[2 * lane + 1] = (uint8_t)(q >> 8);
+                    o[64 + 2 * lane] = (uint8_t)(q >> 16);
+                    o[65 + 2 * lane] = (uint8_t)(q >> 24);
+                }
                 if (lane == 0) *so = sc;
             }
         }
@@ -667,6 +683,8 @@ int launch_pair_one(const TcArgs& g, const PairPlan& pl, cudaStream_t s, const R
     p.npart = pl.npart;
     p.sets = pl.sets;
     p.rope = rope ? *rope : RopeKv{};
+    p.rope_pairs = rope && rv_aligned(rope->cos_t, 4) && rv_aligned(rope->sin_t, 4) && rv_aligned(rope->q_fp8, 2) &&
+                   rv_aligned(rope->k_cache, 2) && rv_aligned(rope->v_cache, 2);
     p.arg_val = g.arg_val;
     p.arg_idx = g.arg_idx;
     p.softcap = g.softcap;

@@ -57,3 +57,37 @@ def test_pair_argmax_equals_argmax_over_logits(orc, M, softcap):
     torch.cuda.synchronize()
     assert gemm.tc_status() == 0
     assert torch.equal(tok, ref) and int(tok[1]) == -1
+
+
+@pytest.mark.parametrize("M", [33, 50, 128])
+@pytest.mark.parametrize("off", [("tables",), ("q8",), ("kc", "vc"), ("tables", "q8", "kc", "vc")])
+def test_pair_qkv_rope_at_odd_addresses(M, off):
+    """RoPE tables at 2-byte and Q / caches at odd addresses: the bytes of the aligned call."""
+    from rvllm_b200 import gemm, launchers
+    heads, kv_heads, HD, K, slots, max_pos = 4, 2, 128, 1024, 3 * M + 5, 96
+    N = (heads + 2 * kv_heads) * HD
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    codes = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    a, w = codes(M, K), codes(N, K)
+    a_s = torch.rand(M, generator=g, device="cuda") * 0.1
+    w_s = torch.rand(N, generator=g, device="cuda") * 0.1
+    ang = torch.rand((max_pos, HD // 2), generator=g, device="cuda") * 6.28
+    pos = torch.randint(0, max_pos, (M,), generator=g, device="cuda", dtype=torch.int32)
+    slot = torch.randperm(slots, generator=g, device="cuda")[:M].to(torch.int32)
+    shift = lambda t, odd: torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape) if odd else t
+
+    def call(off):
+        cos, sin = (shift(f(ang).to(torch.bfloat16), "tables" in off) for f in (torch.cos, torch.sin))
+        out = {k: shift(torch.full(s, 0xAB, dtype=torch.uint8, device="cuda"), k in off)
+               for k, s in dict(q8=(M, heads, HD), kc=(slots, kv_heads, HD), vc=(slots, kv_heads, HD)).items()}
+        out.update({k: torch.zeros(n, device="cuda") for k, n in dict(qs=M * heads, ks=slots * kv_heads, vs=slots * kv_heads).items()})
+        assert all((out[k].data_ptr() & 1) == (k in off) for k in ("q8", "kc", "vc")) and cos.data_ptr() % 4 == 2 * ("tables" in off)
+        assert launchers.qkv_rope_fp8kv(a, w, a_s, w_s, heads, kv_heads, HD, cos, sin, pos, slot, out["q8"], out["qs"], out["kc"],
+                                        out["vc"], out["ks"], out["vs"])
+        torch.cuda.synchronize()
+        assert gemm.tc_status() == 0
+        return out
+
+    want, got = call(()), call(off)
+    assert all(torch.equal(want[k], got[k]) for k in want)
