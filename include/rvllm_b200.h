@@ -238,7 +238,9 @@ int fa_sm89_paged_prefill_fp8(void* q_fp8, void* k_cache_fp8, void* v_cache_fp8,
                               int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                               int num_blocks_total, int window_size_left, void* stream);
 /* Same kernel with the output type selectable and head_dim 64 allowed
- * (PagedDecodeParams, v3/crates/rvllm-attention/src/decode.rs:14-102). */
+ * (PagedDecodeParams, v3/crates/rvllm-attention/src/decode.rs:14-102).  How a sequence's context is cut into chunks, and so
+ * the order of its sums, follows from the tokens it attends, the batch, the head counts and head_dim — not from
+ * max_blocks_per_seq: block tables may be as wide as the longest context there may ever be. */
 int rvllm_paged_decode_fp8_validate(int batch_size, int num_heads, int num_kv_heads, int head_dim,
                                     int block_size, int max_blocks_per_seq, int num_blocks_total,
                                     int window_size_left, float scale);

@@ -70,7 +70,7 @@ void rvllm_paged_decode_cluster_combine(int enabled);
 void rvllm_paged_decode_hint_early_meta(void);
 void rvllm_paged_decode_early_meta(int mode);
 /* The cluster-merged form's own plan: CTAs aimed for (chunks per sequence = ceil(target / (batch * KV heads)), at most
- * 8) and the smallest chunk in tokens; 0 restores the defaults (chunks by a cost model of the shape).  Process-wide. */
+ * 8) and the smallest chunk in tokens; 0 restores the defaults (as many chunks as keep the grid resident at once).  Process-wide. */
 void rvllm_paged_decode_cluster_tune(int target_ctas, int min_chunk_tokens);
 /* Depth of the tcgen05 kernel's K/V ring in 16 KB units (2..8 for head_dim 128, 3..8 for 256);
  * 0 restores the automatic choice.  Tuning aid, process-wide. */

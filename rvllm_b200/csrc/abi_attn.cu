@@ -315,10 +315,10 @@ static int decode_core(const QuantOut& qo, const void* q_fp8, const void* k_cach
             if (cc > 8) cc = 8;
             while (cc > 1 && cc * group * (head_dim + 2) * 4 > rvua::MAX_RECV_BYTES) cc--;
         } else {
-            // tokens a sequence can attend: its block table's capacity, or the window
+            // no sequence attends more than its block table holds, or than the window
             long long len = (long long)block_size * max_blocks_per_seq;
             if (window_size_left >= 0 && window_size_left + 1ll < len) len = window_size_left + 1ll;
-            cc = rvua::pick_cluster_chunks((long long)batch_size * num_kv_heads, (int)(len < (1 << 20) ? len : (1 << 20)), group, head_dim);
+            cc = rvua::pick_cluster_chunks((long long)batch_size * num_kv_heads, len, group, head_dim);
         }
         p.max_chunks = cc;
         p.min_chunk_tokens = g_cluster_min_tokens.load();

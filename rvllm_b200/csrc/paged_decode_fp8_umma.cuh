@@ -866,34 +866,29 @@ template <int HD> inline int pick_units(long long ctas, int extra_bytes = 0) {
     return best;
 }
 
-// Chunks per sequence of the cluster-merged form (1: no split, no cluster) for `units` (sequence, KV head) pairs that attend
-// up to `len` tokens: the cheapest of 1 to 8, in tiles of one CTA.  A CTA is a chain of about 1.5 us per tile with a few
-// CTAs per SM, plus about two tiles of prologue and one of merging.  Half of the cost is what equal contexts take
-// (waves x chunk), half what contexts spread up to `len` take (the mean load of a residency slot and the tail of the
-// longest chunk).  Residency: registers allow 4 / 3 / 2 CTAs of up to 2 / 4 / 8 query heads, the ring 2 and 1 at head_dim
-// 256 and 512.  Measured, us, with the fixed target of 296 CTAs this replaces -> now: 64 sequences of 512 to 32768 tokens,
-// head_dim 256: 1512 -> 1373; 8 of them, head_dim 128: 148 -> 118; 16 of up to 4000 tokens, 64 / 8 heads: 45 -> 33;
-// 4 of up to 100 tokens (no cluster at all now): 6.9 -> 5.2.
-inline int pick_cluster_chunks(long long units, int len, int heads_per_cta, int head_dim) {
+// Chunks per sequence of the cluster-merged form (1: no split, no cluster) for `units` (sequence, KV head) pairs: as many as
+// keep the whole grid resident at once, up to 8, and no more than there are tiles in `capacity` tokens (a sequence is never
+// cut into more chunks than its tiles).  Residency: registers allow 4 / 3 / 2 CTAs of up to 2 / 4 / 8 query heads per SM, the
+// ring 2 and 1 at head_dim 256 and 512.
+//
+// The block table's room only rules out chunks that no sequence can have, so neither the split of a sequence nor the bits of
+// its output depend on it.  It says nothing about the contexts: a table sized for the longest context there may be is the
+// usual case, and a CTA without work is expensive (it keeps its share of the SM until the cluster's last CTA leaves).  A rule
+// that took the room for the contexts' length cut them further where they filled it (64 sequences of 512 to 32768 tokens,
+// head_dim 256: 1.06 to 1.10 times as fast; 8 of them, head_dim 128: 1.10) and lost far more where they did not: 32 of 600 tokens,
+// head_dim 128, with room for 32768, took 57 us instead of 15, 64 of 500 tokens 66 instead of 30.  Measured, us, with a
+// target of 296 CTAs whatever the residency -> now: 8 sequences of 512 to 32768 tokens, head_dim 128: 137 -> 126; 16 of up
+// to 4000 tokens, 64 / 8 heads: 40 -> 32; 4 of 1000 tokens, head_dim 512: 38 -> 22.
+inline int pick_cluster_chunks(long long units, long long capacity, int heads_per_cta, int head_dim) {
     int per_sm = heads_per_cta <= 2 ? 4 : heads_per_cta <= 4 ? 3 : 2;
     if (head_dim == 256 && per_sm > 2) per_sm = 2;
     if (head_dim == 512) per_sm = 1;
-    const long long slots = 148ll * per_sm;
-    const int tiles = (len + TOK - 1) / TOK;
-    int best = 1;
-    double best_cost = 1e300;
-    for (int cc = 1; cc <= 8 && cc <= tiles; cc++) {
-        if (cc > 1 && cc * heads_per_cta * (head_dim + 2) * 4 > MAX_RECV_BYTES) break;
-        const int fixed = cc > 1 ? 3 : 2;
-        const double chunk = (tiles + cc - 1) / cc + fixed;
-        const double even = (double)((units * cc + slots - 1) / slots) * chunk;
-        const double spread = (double)units * (0.6 * tiles + cc * fixed) / slots + 0.5 * chunk;
-        if (even + spread < best_cost) {
-            best_cost = even + spread;
-            best = cc;
-        }
-    }
-    return best;
+    long long cc = 148ll * per_sm / units;
+    const long long tiles = (capacity + TOK - 1) / TOK;
+    if (cc > 8) cc = 8;
+    if (cc > tiles) cc = tiles;
+    while (cc > 1 && cc * heads_per_cta * (head_dim + 2) * 4 > MAX_RECV_BYTES) cc--;
+    return cc > 1 ? (int)cc : 1;
 }
 
 inline int read_status(int* out, bool reset) {

@@ -26,3 +26,19 @@ def test_split_of_long_contexts(orc, HD, ctxs):
     _lib.lib().rvllm_paged_decode_tune(0, 0, 0)
     c = datagen.attention_case(orc, len(ctxs), 8, 4, HD, 16, ctxs, seed=41 + HD)
     assert_close(run_ours(c), run_oracle(orc, c, precise=True))
+
+
+# a block table sized for the longest context there may be: the same chunks, so the same bits, as one of the batch's size
+@pytest.mark.parametrize("HD,batch", [(128, 1), (128, 24), (256, 24), (512, 12), (128, 96)])
+def test_table_capacity_leaves_the_output_alone(orc, HD, batch):
+    import numpy as np
+    from rvllm_b200 import _lib
+    _lib.lib().rvllm_paged_decode_tune(0, 0, 0)
+    ctxs = [[200, 1, 129, 600, 385, 1024][i % 6] + 3 * i for i in range(batch)]
+    c = datagen.attention_case(orc, batch, 8, 4, HD, 16, ctxs, seed=51 + HD)
+    want = run_ours(c)
+    for width in (256, 2048):
+        tables = np.zeros((batch, width), dtype=np.int32)
+        tables[:, :c["max_blocks"]] = c["tables"]
+        got = run_ours(dict(c, tables=tables, max_blocks=width))
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), width
