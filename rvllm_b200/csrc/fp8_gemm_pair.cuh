@@ -649,12 +649,15 @@ inline PairPlan pair_plan(int M, int N, int K, int ranges) {
 
 // Which shapes the pair kernel takes.  Above 32 rows all of them: over the sweep of pair_plan() it is faster than the
 // one-CTA form was from 33 rows on (43008 x 5376: equal up to 64 rows), 1.3 times at 96 rows, 2 to 4 times above 128.  Up
-// to 32 rows only weights of 149 to 295 tiles of 128 rows, which the one-CTA form splits in two and runs in two uneven
-// waves (28672 x 4096 at 8 / 32 rows: 27 / 34 us against 20 / 21); elsewhere there its three small CTAs per SM start faster.
+// to 32 rows only weights that the one-CTA form splits into more CTAs than are resident (three per SM), two uneven waves:
+// 223 to 240 tiles of 128 rows, split in two.  Measured at 1, 8, 16, 17 and 32 rows, K 1024 to 8192, one-CTA time / pair
+// time: there 1.10 to 1.67 (28672 x 4096: 26.3 / 21.8 us at one row, 32.7 / 22.7 at 32).  Next to it the one-CTA form wins
+// or ties, its three small CTAs per SM start faster: 149 to 222 tiles 0.77 to 1.03 up to 16 rows (0.86 to 1.3 at 17 to 32,
+// where the short K gain), 241 to 295 tiles, not split, 0.75 to 1.13, mostly 0.95 to 1.02.
 inline bool prefer_pair(int M, int N, int K) {
     if (K % 16 != 0) return false;
-    const int tiles = (N + TILE_W - 1) / TILE_W;
-    return M > 32 || (tiles > 148 && tiles < 296);
+    const int tiles = (N + TILE_W - 1) / TILE_W, splits = splits_of(tiles, (K + BK - 1) / BK, SPLIT_TARGET);
+    return M > 32 || (splits > 1 && tiles * splits > 3 * 148);
 }
 
 template <int EPI, typename OutT>

@@ -1117,6 +1117,13 @@ int launch_epi(const TcArgs& g, int splits, int stages, cudaStream_t s) {
 
 // Split-K factor: aim for ~2.5 CTAs per SM (measured best on the decode shapes: 64 weight
 // tiles -> 6 splits, 42 tiles -> 8, 336 tiles -> 1), keeping at least four K blocks per CTA.
+constexpr int SPLIT_TARGET = 360;
+inline int splits_of(int tiles, int kblocks, int target) {
+    int s = (target + tiles / 2) / tiles;
+    if (s > 8) s = 8;
+    while (s > 1 && kblocks / s < 4) s--;
+    return s < 1 ? 1 : s;
+}
 inline int pick_splits(int M, int N, int K, int bn) {
     const int tiles = ((N + TILE_W - 1) / TILE_W) * ((M + bn - 1) / bn);
     const int kblocks = (K + BK - 1) / BK;
@@ -1124,12 +1131,8 @@ inline int pick_splits(int M, int N, int K, int bn) {
         const long long e = tune().split_for[i].load();
         if (e != 0 && (e >> 40) == N && ((e >> 8) & 0xffffffffll) == K) return (int)(e & 0xff);
     }
-    const int target = tune().split_target.load() > 0 ? tune().split_target.load() : 360;
-    int s = (target + tiles / 2) / tiles;
-    if (s > 8) s = 8;
-    while (s > 1 && kblocks / s < 4) s--;
-    if (s < 1) s = 1;
-    return s;
+    const int target = tune().split_target.load();
+    return splits_of(tiles, kblocks, target > 0 ? target : SPLIT_TARGET);
 }
 
 // Ring depth: a shallow ring lets three CTAs share an SM, so one CTA's prologue / epilogue overlaps
