@@ -133,17 +133,22 @@ _native = None
 
 def native():
     """The CPython module of the launch entry points (``csrc/py_launch.cpp``): the library's functions without the cost
-    of a ctypes call.  Missing is a hard error, as for the library itself."""
+    of a ctypes call.  Missing is a hard error, as for the library itself; so is a module built for another torch, whose
+    tensors it would read through the wrong class layout."""
     global _native
     if _native is None:
         lib()
-        import torch  # noqa: F401  (the module reads tensors through torch's own libraries, which must be loaded)
+        import torch  # (the module reads tensors through torch's own libraries, which must be loaded)
 
         try:
             from . import _native as module
         except ImportError as e:
             raise RvllmError(E_ARTIFACT, "load", f"rvllm_b200/_native.so cannot be loaded ({e}); build it with "
                                                  "`python -m rvllm_b200.build`") from e
+        built_for = getattr(module, "torch_version", None)
+        if built_for != str(torch.__version__):
+            raise RvllmError(E_ARTIFACT, "load", f"rvllm_b200/_native.so was built for torch {built_for}, this is "
+                                                 f"{torch.__version__}; rebuild it with `python -m rvllm_b200.build`")
         _native = module
     return _native
 

@@ -122,15 +122,22 @@ def build_library(force=False, verbose=False):
 def build_native(force=False):
     """The CPython module of the launch entry points, linked against the library beside it."""
     src = os.path.join(CSRC, "py_launch.cpp")
-    if force or _newer(NATIVE, [src, os.path.join(os.path.dirname(HERE), "include", "rvllm_b200.h"), LIB]):
-        import torch
+    import torch
+
+    stamp = os.path.join(OBJ, "native_torch_version")  # the torch the module on disk was compiled against
+    same_torch = os.path.exists(stamp) and open(stamp).read() == str(torch.__version__)
+    if force or not same_torch or _newer(NATIVE, [src, os.path.join(os.path.dirname(HERE), "include", "rvllm_b200.h"), LIB]):
         from torch.utils import cpp_extension
 
+        os.makedirs(OBJ, exist_ok=True)
         includes = [x for d in [sysconfig.get_paths()["include"], *cpp_extension.include_paths()] for x in ("-isystem", d)]
         # (torch's libraries are in the process before the module is: no path to them is recorded)
         _run(["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+              f'-DRVLLM_TORCH_VERSION="{torch.__version__}"',
               *includes, src, "-o", NATIVE, "-L", HERE, "-l:librvllm_b200.so", "-L", cpp_extension.library_paths()[0],
               "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-Wl,-rpath,$ORIGIN"])
+        with open(stamp, "w") as f:
+            f.write(str(torch.__version__))
     return NATIVE
 
 

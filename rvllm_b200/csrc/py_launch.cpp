@@ -185,5 +185,11 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Launch entry points o
 
 PyMODINIT_FUNC PyInit__native(void) {
     g_data_ptr = PyUnicode_InternFromString("data_ptr");
-    return g_data_ptr ? PyModule_Create(&g_module) : nullptr;
+    PyObject* m = g_data_ptr ? PyModule_Create(&g_module) : nullptr;
+    // The class layouts inlined above are those of the torch this was compiled against; the Python side refuses another.
+    if (m && PyModule_AddStringConstant(m, "torch_version", RVLLM_TORCH_VERSION) != 0) {
+        Py_DECREF(m);
+        m = nullptr;
+    }
+    return m;
 }

@@ -143,6 +143,19 @@ def test_missing_library_is_a_hard_error(monkeypatch, tmp_path):
         _lib.lib()
 
 
+def test_native_module_for_another_torch_is_a_hard_error(monkeypatch):
+    """The module reads tensors through torch's class layouts as they were at compile time."""
+    import torch
+
+    from rvllm_b200 import _lib
+    assert _lib.native().torch_version == str(torch.__version__)
+    monkeypatch.setattr(_lib, "_native", None)
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    with pytest.raises(_lib.RvllmError) as e:
+        _lib.native()
+    assert e.value.code == _lib.E_ARTIFACT
+
+
 def test_build_register_budget_check():
     """The build refuses a kernel that counts on three CTAs per SM when ptxas gave it more than 96 registers."""
     from rvllm_b200 import build
