@@ -24,11 +24,35 @@ def test_pair_gemm(orc, M, N, K, mode):
 
 
 # more tiles than pairs: the persistent loop, both accumulators, ring wrap-around
-@pytest.mark.parametrize("M,N,K", [(300, 43008, 576), (2048, 5376, 320), (8, 28672, 192)])
+@pytest.mark.parametrize("M,N,K", [(300, 43008, 576), (2048, 5376, 320), (8, 28672, 192), (8, 28672, 1024)])
 def test_pair_gemm_many_tiles(orc, M, N, K):
     a, a_s, w, w_s, cols, want = case(orc, M, N, K, seed=10, n_cols=64)
     out = run(TC, a, a_s, w, w_s, torch.bfloat16)
     close(out.float().cpu().numpy()[:, cols], want)
+
+
+# the sum over K does not depend on the batch up to 128 rows, so neither do a row's bytes: the one-CTA form's batch tiles of
+# 16 and 32 rows, the pair form's one and two K ranges per pair; residual and plain, and a shape the pair form takes throughout
+@pytest.mark.parametrize("N,K,residual", [(8192, 5376, False), (5376, 4096, True), (43008, 5376, False), (5376, 21504, True),
+                                          (28672, 4096, False)])
+def test_a_rows_bytes_do_not_depend_on_the_batch(N, K, residual):
+    from rvllm_b200 import gemm
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N + K)
+    codes = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    A, W = codes(128, K), codes(N, K)
+    AS, WS = torch.rand(128, generator=g, device="cuda"), torch.rand(N, generator=g, device="cuda")
+    R = torch.randn((128, N), generator=g, device="cuda").bfloat16() if residual else None
+
+    def call(M):
+        out = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+        gemm.fp8_gemm_channelscale(out, A[:M], W, AS[:M], WS, residual=R[:M] if residual else None, impl=TC)
+        return out
+
+    full = call(128)
+    for M in (1, 16, 17, 32, 33, 64, 65, 127):
+        assert torch.equal(call(M), full[:M]), M
+    assert gemm.tc_status() == 0
 
 
 @pytest.mark.parametrize("M", [33, 130, 300])

@@ -40,6 +40,30 @@ def test_norm(orc, hidden, add):
         assert (out.cpu().numpy() != wb).mean() < 5e-3
 
 
+# an address the vector form does not take selects the reference geometry: same codes, scales and residual, bit for bit
+@pytest.mark.parametrize("hidden", [8, 328, 1000, 1024, 1032, 5376, 8192, 8200])
+@pytest.mark.parametrize("add", [False, True])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_norm_equals_reference_geometry(hidden, add, dt):
+    from rvllm_b200.launchers import FusedAddRmsnormFp8QuantLaunch, FusedRmsnormFp8QuantLaunch
+    T = 5
+    x, r, g = _rand(T, hidden, dt=dt), _rand(T, hidden, dt=dt, seed=1), _rand(hidden, dt=dt, seed=2)
+
+    def call(odd):
+        at = lambda t: torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape) if odd else t.clone()
+        xx, res = at(x), at(r)
+        assert (xx.data_ptr() % 16 != 0) == odd
+        out = torch.empty((T, hidden), dtype=torch.uint8, device="cuda")
+        sc = torch.empty(T, dtype=torch.float32, device="cuda")
+        if add:
+            FusedAddRmsnormFp8QuantLaunch(T, hidden, 1e-6).launch(out, sc, res, xx, res, g)
+        else:
+            FusedRmsnormFp8QuantLaunch(T, hidden, 1e-6).launch(out, sc, xx, g)
+        return out, sc.view(torch.int32), res.view(torch.int16)
+
+    assert all(torch.equal(a, b) for a, b in zip(call(False), call(True)))
+
+
 @pytest.mark.parametrize("dim", [8, 264, 1024, 1032, 4096, 32768, 32776])
 def test_quant(orc, dim):
     from rvllm_b200.launchers import QuantizeFp8PerTokenLaunch
