@@ -126,7 +126,8 @@ int rvllm_fp8_gemm_tc_status(int* status, int reset);
  * [M, (heads + 2*kv_heads)*128] 16-bit buffer followed by rvllm_rope_fp8kv_launch with rotary_dim =
  * head_dim, bit for bit, without the buffer and without the second launch.  head_dim must be 128 (one
  * 128-row weight tile is one head) and M <= 128; returns RVLLM_E_UNSUPPORTED for shapes it does not
- * take (use the two calls).  dtype: the 16-bit type of the implied intermediate and of the tables. */
+ * take (use the two calls).  dtype: the 16-bit type of the implied intermediate and of the tables, which are 2-byte
+ * aligned; a_fp8 and w_fp8 are 16-byte aligned; Q and the caches may stand at any address. */
 int rvllm_fp8_gemm_qkv_rope_fp8kv(const void* a_fp8, const void* w_fp8, const float* a_scale, const float* w_scale, int M,
                                   int K, int heads, int kv_heads, int head_dim, int dtype, void* q_fp8, float* q_scale,
                                   void* k_cache, void* v_cache, float* k_scale_cache, float* v_scale_cache,
@@ -250,10 +251,11 @@ int rvllm_paged_decode_max_chunks(int batch_size, int num_kv_heads);
  * head, pages of 8..128 tokens that divide 128).  Its waits on mbarriers are bounded; this reads
  * (and optionally clears) the word that records the first wait that gave up: 0 = none. */
 int rvllm_paged_decode_tc_status(int* status, int reset);
-/* Which main kernel a launch of this shape runs (1 = both products on the FP32 pipes, 2 = scores on
+/* Which main kernel takes a shape in every form of the call (1 = both products on the FP32 pipes, 2 = scores on
  * mma.sync FP8 tensor cores and P.V on the FP32 pipes, 3 = both products on mma.sync, 4 = tcgen05 /
- * TMEM / TMA: 4 where the shape allows it, else 3, else 2); negative on bad arguments.  head_dim 512 is reported as 2
- * although its plain form runs on 4: it leaves no per-KV-head maxima, which is what callers ask this for. */
+ * TMEM / TMA: 4 where the shape allows it, else 3, else 2); negative on bad arguments.  4 therefore also says that
+ * rvllm_paged_decode_fp8_amax takes the shape.  At head_dim 512 that call is refused and the answer is 2; a call without
+ * the maxima runs on 4 there all the same (heads and pages as for 4). */
 int rvllm_paged_decode_kernel_for(int num_heads, int num_kv_heads, int head_dim, int block_size, int num_blocks_total);
 int rvllm_paged_decode_fp8(const void* q_fp8, const void* k_cache_fp8, const void* v_cache_fp8, void* output,
                            int out_dtype, const int32_t* block_tables, const int32_t* context_lens,

@@ -24,8 +24,10 @@ void rvllm_b200_set_pdl(int enabled);
 int rvllm_b200_get_pdl(void);
 
 /* Overrides of the tcgen05 kernel's automatic choices, for tuning runs: TMA ring depth
- * (2..8) and split-K factor (1..8); 0 restores the automatic choice.  Process-wide.  They and the two hooks below
- * concern launches of up to 32 rows: the CTA-pair kernel that takes larger ones has its own plan. */
+ * (2..8) and split-K factor (1..8); 0 restores the automatic choice.  Process-wide.  These two concern launches of up
+ * to 32 rows, as the form of the reduction below does: the CTA-pair kernel that takes larger ones has its own plan.  (It
+ * adds the K ranges of the one-CTA plan, so that a row's bytes do not depend on the batch up to 128 rows; while `splits`
+ * is set, launches of up to 32 rows round in another order than it.) */
 void rvllm_fp8_gemm_tc_tune(int stages, int splits);
 /* Form of the split-K reduction inside a cluster: 0 automatic (partials are pushed into the finishing CTA's receive
  * buffer and every sender arrives on the owner's mbarrier), 1 always pull out of the peers' rings, 2 the same as 0,
@@ -34,7 +36,7 @@ void rvllm_fp8_gemm_tc_tune(int stages, int splits);
  * results are bitwise equal (tested). */
 void rvllm_fp8_gemm_tc_reduce(int mode);
 /* CTAs a split-K launch aims for (splits = round(target / weight tiles), at most 8, at least 4 K blocks each);
- * 0 restores the built-in 360.  Process-wide. */
+ * 0 restores the built-in 360.  Process-wide.  Up to 128 rows: the CTA-pair kernel's K ranges follow it. */
 void rvllm_fp8_gemm_tc_split_target(int ctas);
 /* Timing aid of the tcgen05 GEMM: while a device buffer of `slots` x 16 u64 is set, every launch takes the next row
  * (launch order, modulo `slots`; the count restarts with this call) and leaves, for each of 8 points, the
@@ -45,7 +47,7 @@ void rvllm_fp8_gemm_tc_split_target(int ctas);
  * The stamps exist only in a library built with RVLLM_TC_TRACE=1 (they cost the decode step 1.2 % even when off);
  * otherwise setting a buffer returns RVLLM_E_UNSUPPORTED. */
 int rvllm_fp8_gemm_tc_trace(void* device_u64_buffer, int slots);
-/* Split-K factor of one weight shape [N, K], four slots; splits 0 clears the slot. */
+/* Split-K factor of one weight shape [N, K], four slots; splits 0 clears the slot.  Up to 128 rows, as above. */
 void rvllm_fp8_gemm_tc_split_for(int slot, int N, int K, int splits);
 
 /* Overrides for tuning runs (0 restores the default): CTAs the grid aims for, the fewest tokens

@@ -87,7 +87,7 @@ int launch_act_stream(uint32_t rows, int inter, uint8_t* out, float* scale, cons
     static RvDeviceOnce once;
     auto kern = rvrow::act_mul_quant_stream_kernel<ACT, T, NC>;
     if (rv_allow_smem(once, kern, 220 * 1024)) return -1;
-    rv_launch(kern, dim3(rv_umin(rows, 148)), dim3(1024), (size_t)8 * inter, s, dim3(1, 1, 1), out, scale, (const T*)gate_up, inter, (int)rows);
+    rv_launch(kern, dim3(rv_umin(rows, rv::SMS)), dim3(1024), (size_t)8 * inter, s, dim3(1, 1, 1), out, scale, (const T*)gate_up, inter, (int)rows);
     return 0;
 }
 

@@ -87,7 +87,7 @@ int launch_stream_epi(const GemmArgs& g, const rvgemm::StreamParams& p, int spli
 int stream_splits(int M, int N, int K, int mblocks) {
     (void)M;
     const int tiles = ((N + rvgemm::TILE_N - 1) / rvgemm::TILE_N) * mblocks;
-    int s = (2 * 148 + tiles - 1) / tiles;
+    int s = (2 * rv::SMS + tiles - 1) / tiles;
     const int chunks = K / rvgemm::CHUNK;
     while (s > 1 && chunks / (s * rvgemm::K_WARPS) < 2) s--;
     if (s < 1) s = 1;

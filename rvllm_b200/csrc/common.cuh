@@ -11,6 +11,9 @@
 
 namespace rv {
 
+// SMs of a B200.  Grids and plans are sized for it; on a part with fewer SMs they are correct but no longer the best.
+constexpr int SMS = 148;
+
 // ---- 16-bit activation types ------------------------------------------------------
 template <typename T> struct T16;
 template <> struct T16<__half> {

@@ -355,7 +355,7 @@ int enqueue_step(rvllm_stack* s, int* launches, bool chained = false) {
         }
         x_ready = false;
         // QKV projection, RoPE, Q quantisation and the paged KV write: one launch where the library
-        // takes the shape (head_dim 128, batch <= 32, tensor-core GEMM), else the GEMM and the RoPE kernel
+        // takes the shape (head_dim 128, batch <= 128, tensor-core GEMM), else the GEMM and the RoPE kernel
         int fused = RVLLM_E_UNSUPPORTED;
         if (!on(2)) fused = RVLLM_OK, n--;  // (left out: timing aid)
         else if (L.head_dim == 128 && c.gemm_impl != 1)

@@ -25,10 +25,10 @@
 // split-K factor the one-CTA form's plan gives the shape, so that a batch decodes to the same bytes whichever kernel
 // takes it (a decoder stack amplifies the rounding of another order to the size of its FP8 steps within a few layers).
 //
-// Large batches are bound by the tensor pipe and the power cap, small ones by the weights' stream.  Measured, us, one-CTA
-// form (256-row batch tiles, pull reduction) -> pairs: [8192 x 5376] at M = 500 / 2048: 30 / 125 -> 22 / 66; [43008 x 5376]
-// 162 / 725 -> 92 / 305 (3.1 PFLOP/s); [5376 x 21504] + residual 133 / 517 -> 53 / 190; at M = 128 the four projections
-// 20 / 17 / 48 / 33 -> 13 / 11 / 45 / 26.
+// Large batches are bound by the tensor pipe and the power cap, small ones by the weights' stream.  Measured, us, a one-CTA
+// form with 256-row batch tiles and a pull reduction against pairs: [8192 x 5376] at M = 500 / 2048: 30 / 125 against 22 / 66;
+// [43008 x 5376] 162 / 725 against 92 / 305 (3.1 PFLOP/s); [5376 x 21504] + residual 133 / 517 against 53 / 190; at M = 128
+// the four projections 20 / 17 / 48 / 33 against 13 / 11 / 45 / 26.
 //
 // Every wait is bounded and reports through the status word of fp8_gemm_tc.cuh.
 #pragma once
@@ -40,6 +40,7 @@ using namespace rvtc;
 
 constexpr int PAIR_THREADS = 384;
 constexpr int PAIR_EPI_WARP0 = 4, PAIR_EPI_WARPS = 8;
+constexpr int PAIRS = rv::SMS / 2;
 constexpr int PAIR_MAX_STAGES = 8, PAIR_HEADER = 4096;
 
 struct PairParams {
@@ -169,7 +170,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         for (int t = cluster_id; t < p.tiles && alive; t += clusters) {
             const int n0 = (t / p.nb) * 256 + (int)half * TILE_W, m0 = (t % p.nb) * BN + (int)half * b_rows;
             // Weights never depend on the previous kernel: the first ring of weight tiles goes out before the wait
-            // for it, the activation tiles of those stages follow.
+            // for it, the activation tiles of those stages follow.  (That is early only where this CTA found its SM empty:
+            // its shared memory is the whole SM's, so it never starts beside a CTA of the kernel before it.)
             const int pre = waited ? 0 : (nkb < STAGES ? nkb : STAGES);
             if (!waited) {
                 for (int i = 0; i < pre; i++) {
@@ -616,7 +618,6 @@ inline int pair_recv_slots(int V, int S) {
 // sweep of 16 weight shapes (512 x 512 to 43008 x 5376) and 20 batch sizes (4 to 2048): on it the choice is 1.4 % off the
 // best candidate on average, 23 % at worst (launches of 6 us).
 inline PairPlan pair_plan(int M, int N, int K, int ranges) {
-    constexpr int PAIRS = 74;
     const int nw = (N + 255) / 256, kblocks = (K + BK - 1) / BK, nb0 = (M + 255) / 256;
     PairPlan best = {};
     double best_cost = 0.0;
@@ -657,7 +658,7 @@ inline PairPlan pair_plan(int M, int N, int K, int ranges) {
 inline bool prefer_pair(int M, int N, int K) {
     if (K % 16 != 0) return false;
     const int tiles = (N + TILE_W - 1) / TILE_W, splits = splits_of(tiles, (K + BK - 1) / BK, SPLIT_TARGET);
-    return M > 32 || (splits > 1 && tiles * splits > 3 * 148);
+    return M > 32 || (splits > 1 && tiles * splits > 3 * rv::SMS);
 }
 
 template <int EPI, typename OutT>
@@ -694,7 +695,7 @@ int launch_pair_one(const TcArgs& g, const PairPlan& pl, cudaStream_t s, const R
     const int stage_bytes = TILE_W * BK + pl.bn / 2 * BK;
     p.stages = (SMEM - 1024 - PAIR_HEADER - pair_extra_bytes(EPI)) / stage_bytes;
     if (p.stages > PAIR_MAX_STAGES) p.stages = PAIR_MAX_STAGES;
-    const int clusters = pl.splits > 1 ? pl.tiles : (pl.tiles < 74 ? pl.tiles : 74);
+    const int clusters = pl.splits > 1 ? pl.tiles : (pl.tiles < PAIRS ? pl.tiles : PAIRS);
     if (rv_launch(kern, dim3(clusters * 2 * pl.splits), dim3(PAIR_THREADS), SMEM, s, dim3(2 * pl.splits, 1, 1), mw, ma, p) !=
         cudaSuccess) {
         cudaGetLastError();

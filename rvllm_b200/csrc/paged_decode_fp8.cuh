@@ -29,7 +29,7 @@ constexpr int THREADS = 256;
 constexpr int WARPS = THREADS / 32;
 constexpr int MIN_CHUNK_TOKENS = 256;
 constexpr int MAX_CHUNKS = 32;
-constexpr int TARGET_CTAS = 148 * 2;  // measured: more, smaller CTAs only add merge work
+constexpr int TARGET_CTAS = rv::SMS * 2;  // measured: more, smaller CTAs only add merge work
 constexpr int DEPTH = 8;            // cp.async rounds in flight per warp
 constexpr int STAGE_BYTES = 1088;   // 32 lanes x 16 B of K, the same of V, 8 + 8 row scales
 constexpr int TBL_MAX = 2048;       // block-table entries staged in shared memory per CTA

@@ -856,7 +856,7 @@ template <int HD> inline int pick_units(long long ctas, int extra_bytes = 0) {
     int best = cand[0].units;
     double best_cost = 1e300;
     for (int i = 0; i < n; i++) {
-        const long long slots = ((228 * 1024) / (C::smem_bytes(cand[i].units) + extra_bytes + 1024)) * 148ll;
+        const long long slots = ((228 * 1024) / (C::smem_bytes(cand[i].units) + extra_bytes + 1024)) * (long long)rv::SMS;
         const double cost = (double)((ctas + slots - 1) / slots) * cand[i].wave;
         if (cost < best_cost) {
             best_cost = cost;
@@ -877,13 +877,13 @@ template <int HD> inline int pick_units(long long ctas, int extra_bytes = 0) {
 // that took the room for the contexts' length cut them further where they filled it (64 sequences of 512 to 32768 tokens,
 // head_dim 256: 1.06 to 1.10 times as fast; 8 of them, head_dim 128: 1.10) and lost far more where they did not: 32 of 600 tokens,
 // head_dim 128, with room for 32768, took 57 us instead of 15, 64 of 500 tokens 66 instead of 30.  Measured, us, with a
-// target of 296 CTAs whatever the residency -> now: 8 sequences of 512 to 32768 tokens, head_dim 128: 137 -> 126; 16 of up
-// to 4000 tokens, 64 / 8 heads: 40 -> 32; 4 of 1000 tokens, head_dim 512: 38 -> 22.
+// target of 296 CTAs whatever the residency / with this rule: 8 sequences of 512 to 32768 tokens, head_dim 128: 137 / 126;
+// 16 of up to 4000 tokens, 64 / 8 heads: 40 / 32; 4 of 1000 tokens, head_dim 512: 38 / 22.
 inline int pick_cluster_chunks(long long units, long long capacity, int heads_per_cta, int head_dim) {
     int per_sm = heads_per_cta <= 2 ? 4 : heads_per_cta <= 4 ? 3 : 2;
     if (head_dim == 256 && per_sm > 2) per_sm = 2;
     if (head_dim == 512) per_sm = 1;
-    long long cc = 148ll * per_sm / units;
+    long long cc = (long long)rv::SMS * per_sm / units;
     const long long tiles = (capacity + TOK - 1) / TOK;
     if (cc > 8) cc = 8;
     if (cc > tiles) cc = tiles;

@@ -3,9 +3,9 @@
 //
 // What bounds the reference geometry at prefill-sized row counts is not bandwidth: 1024 threads per row hold one vector
 // each, spend their time in four block-wide barriers, and two such blocks fill an SM; a (token, head) block of 64 threads
-// per RoPE head does 500 bytes of work per launch slot.  Measured on [1000 x 5376 / 21504], us, before -> now:
-// add + norm + quant 17.6 -> 7.0, RoPE + KV write 33.9 -> 10.7, act + quant 47.3 -> 28.4, per-token quant (4096) 8.0 -> 3.1;
-// on 32 rows the norm 4.1 -> 2.9.
+// per RoPE head does 500 bytes of work per launch slot.  Measured on [1000 x 5376 / 21504], us, reference geometry / here:
+// add + norm + quant 17.6 / 7.0, RoPE + KV write 33.9 / 7.4 (16-byte loads, see its launcher), act + quant 47.3 / 28.4,
+// per-token quant (4096) 8.0 / 3.1; on 32 rows the norm 4.1 / 2.9.
 //
 // (What a preceding kernel wrote is read with plain loads: see rv::ldg128.)
 #pragma once
