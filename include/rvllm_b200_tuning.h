@@ -62,9 +62,10 @@ void rvllm_paged_decode_tune(int target_ctas, int min_chunk_tokens, int variant)
  * combine kernel, as the other variants do.  Process-wide. */
 void rvllm_paged_decode_cluster_combine(int enabled);
 /* Early metadata: the tcgen05 attention kernel reads context lengths and block tables, and fetches every K / V tile but
- * the last of a sequence, without waiting for the kernel before it in the stream (programmatic dependent launch); only
- * Q, the last tile and the scales wait.  Legal only for a caller whose context lengths, block tables and older cache
- * rows were complete before that kernel could start — the decode stack's graph qualifies: its bookkeeping for a step is
+ * the last of a sequence, without waiting for the kernel before it in the stream (programmatic dependent launch); so
+ * are, in the cluster-merged form, the scales of a chunk's first tile but the newest token's.  Q, the last tile and the
+ * other scales wait.  Legal only for a caller whose context lengths, block tables and older cache rows, with their
+ * scales, were complete before that kernel could start — the decode stack's graph qualifies: its bookkeeping for a step is
  * written by the last kernel of the step before, and consecutive graph launches do not overlap.
  * `rvllm_paged_decode_hint_early_meta()`: one-shot, calling thread only — the next decode-attention launch made from
  * this thread runs in that mode.  `rvllm_paged_decode_early_meta(mode)`: process-wide override, 0 = as hinted

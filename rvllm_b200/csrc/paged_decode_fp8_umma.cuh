@@ -320,14 +320,24 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
 
     const int nh = group < GT ? group : GT;  // query heads of this KV head (the launcher guarantees group <= GT)
     int ph_first = 0;
+    float ks_first = 0.0f, vs_first = 0.0f;
+    bool scales_first = false;
     if (warp != 0) {
         // The producer warp goes straight to its loads; the other five warps stage Q meanwhile.
+        if (active && warp >= 2) {  // softmax warps: the block of this thread's first token, on its way while Q is staged
+            const int tok = tile0 + ((warp & 3) * 32 + lane);
+            if (tok >= t_begin && tok < t_end) ph_first = block_of(tok);  // (early: block tables do not wait)
+            // Nor do the scales of older tokens.  Only in the cluster form, whose grid is resident at once: a CTA of a later
+            // wave has nothing to wait for, and there this chain would hold back the staging of Q.
+            if (CL && early && tok >= t_begin && tok < t_end && tok + 1 < ctx && (unsigned)ph_first < (unsigned)p.num_blocks_total) {
+                const size_t sidx = ((size_t)ph_first * bs + (tok % bs)) * p.kv_heads + kvh;
+                if (p.k_scale_cache) ks_first = p.k_scale_cache[sidx];
+                if (p.v_scale_cache) vs_first = p.v_scale_cache[sidx];
+                scales_first = true;
+            }
+        }
         if (early) rv::pdl_wait();  // Q, and the newest token's scales, come from the preceding kernel
         if (active) {
-            if (warp >= 2) {  // softmax warps: the block of this thread's first token, on its way while Q is staged
-                const int tok = tile0 + ((warp & 3) * 32 + lane);
-                if (tok >= t_begin && tok < t_end) ph_first = block_of(tok);
-            }
             // Q codes of the KV head's query heads -> B operand panels (K-major, swizzled by hand)
             for (int i = tid - 32; i < nh * (HD / 16); i += THREADS - 32) {
                 const int n = i / (HD / 16), c = i % (HD / 16), h = c >> 3, cc = c & 7;
@@ -523,8 +533,9 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                     ph = 0;
                 }
                 const size_t sidx = ((size_t)ph * bs + (tok % bs)) * p.kv_heads + kvh;
-                if (k_perslot) ks = p.k_scale_cache[sidx];
-                if (v_perslot) vs = p.v_scale_cache[sidx];
+                const bool have = CL && i == 0 && scales_first;
+                if (k_perslot) ks = have ? ks_first : p.k_scale_cache[sidx];
+                if (v_perslot) vs = have ? vs_first : p.v_scale_cache[sidx];
             }
         };
         bool valid_n, alive = true;
