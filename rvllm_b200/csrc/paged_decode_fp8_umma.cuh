@@ -93,6 +93,28 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
+// The pages of one panel of a tile, page j's first slot in lane j.  One elected lane issues them out of a loop of the whole warp,
+// its operands in uniform registers: lanes that issue side by side are served one after another, 120 cycles each, against 70 here.
+// A tile of head_dim 256 in 16-token pages has 32 of these instructions, which made the producer the kernel's longest chain.
+__device__ __forceinline__ void load_pages(uint8_t* dst, int page_bytes, const CUtensorMap* map, int x, int head, int slots, int np, bool one,
+                                           uint64_t* bar) {
+    int j = 0;
+#pragma unroll 1
+    for (; j + 4 <= np; j += 4) {
+        int z[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) z[k] = __shfl_sync(0xffffffffu, slots, j + k);
+        if (one) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) tma_load_3d(dst + (size_t)(j + k) * page_bytes, map, x, head, z[k], bar);
+        }
+    }
+#pragma unroll 1
+    for (; j < np; j++) {
+        const int z = __shfl_sync(0xffffffffu, slots, j);
+        if (one) tma_load_3d(dst + (size_t)j * page_bytes, map, x, head, z, bar);
+    }
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t* holder, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)), "r"(cols)
                  : "memory");
@@ -201,7 +223,7 @@ __device__ __forceinline__ void split3(float x, uint8_t& hi, uint8_t& mid, uint8
 // CL: the cluster-merged split-KV form (Params::cluster_combine), an instantiation of its own: the plain one keeps
 // its 64 registers — five CTAs of the shallowest ring share an SM (30 warps), which a batch-128 launch counts on.
 template <int HD, int GT, typename OutT, bool CL>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(THREADS, !CL && HD == 128 && GT <= 2 ? 5 : 1)
 paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, Params p,
                              int nunits) {
     static_assert(HD == 128 || HD == 256 || HD == 512, "one, two or four 128-byte panels per cache row");
@@ -356,6 +378,7 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
         // cost ~2 us per tile that way, more than the loads themselves).
         if (ntiles > 0) {
             const int ppt = TOK / bs;  // pages per tile (<= 16)
+            const bool one = rv::elect_one();
             bool alive = true, bad_page = false;
             int slot = 0, use = 0;  // ring position of the next unit (kept incrementally: NUNITS is a run-time value)
             for (int i = 0; i < ntiles && alive; i++) {
@@ -368,16 +391,11 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 if (lane < np) z = phys_of(tok_tile + lane * bs, bad_page) * bs;
 #pragma unroll 1
                 for (int u = 0; u < UPT && alive; u++) {
-                    if (use > 0) {
-                        if (lane == 0) alive = mbar_wait(empty + slot, (uint32_t)(use - 1) & 1u, 1);
-                        alive = __shfl_sync(0xffffffffu, (int)alive, 0) != 0;
-                    }
+                    if (use > 0) alive = __all_sync(0xffffffffu, mbar_wait(empty + slot, (uint32_t)(use - 1) & 1u, 1)) != 0;
                     if (!alive) break;
-                    if (lane == 0) mbar_expect_tx(full + slot, (uint32_t)(np * bs * PANEL));
-                    __syncwarp();
-                    if (lane < np)
-                        tma_load_3d(ring + (size_t)slot * UNIT + (size_t)lane * bs * PANEL, u < HALVES ? &map_k : &map_v,
-                                    (u % HALVES) * PANEL, kvh, z, full + slot);
+                    if (one) mbar_expect_tx(full + slot, (uint32_t)(np * bs * PANEL));
+                    load_pages(ring + (size_t)slot * UNIT, bs * PANEL, u < HALVES ? &map_k : &map_v, (u % HALVES) * PANEL, kvh, z, np, one,
+                               full + slot);
                     if (++slot == NUNITS) {
                         slot = 0;
                         use++;
