@@ -10,6 +10,7 @@
 #include "host_util.h"
 #include "paged_decode_fp8_tc.cuh"
 #include "paged_decode_fp8_umma.cuh"
+#include "paged_decode_fp8_items.cuh"
 
 // Tuning overrides (declared in rvllm_b200_tuning.h).  Atomics: a setter racing a launch on another thread
 // yields the old or the new value, never a torn one; a workspace query and its launch must still not
@@ -136,7 +137,7 @@ int launch_umma_form(const rvattn::Params& p, cudaStream_t s) {
     // cluster-combine form: the chunks of a (sequence, KV head) are one cluster, the receive area sits behind the rest
     // (and counts when the ring depth is chosen: a third of the footprint at eight chunks)
     const size_t recv = p.cluster_combine ? (size_t)C::recv_bytes(p.max_chunks, p.heads / p.kv_heads) : 0;
-    int units = ring > 0 ? ring : rvua::pick_units<HD>((long long)p.kv_heads * p.max_chunks * p.batch, (int)recv);
+    int units = ring > 0 ? ring : rvua::pick_units<C>((long long)p.kv_heads * p.max_chunks * p.batch, (int)recv);
     if (units < C::MIN_UNITS) units = C::MIN_UNITS;
     if (units > C::MOST_UNITS) units = C::MOST_UNITS;
     while (units > C::MIN_UNITS && C::smem_bytes(units) + recv > (size_t)C::smem_bytes(C::MOST_UNITS)) units--;
@@ -146,7 +147,33 @@ int launch_umma_form(const rvattn::Params& p, cudaStream_t s) {
 }
 
 template <int HD, int GT, typename OutT>
+int launch_items(const rvattn::Params& p, cudaStream_t s) {
+    CUtensorMap mk, mv, mq;
+    const long long slots = (long long)p.num_blocks_total * p.block_size;
+    const int group = p.heads / p.kv_heads;
+    if (!rvua::cache_map(&mk, p.k_cache, slots, p.kv_heads, HD, p.block_size) ||
+        !rvua::cache_map(&mv, p.v_cache, slots, p.kv_heads, HD, p.block_size) ||
+        !rvua::cache_map(&mq, p.q, (long long)p.batch * p.heads, 1, HD, group))  // Q: rows of a KV head's query heads
+        return rv_fail(RVLLM_E_LAUNCH, "cuTensorMapEncodeTiled failed for the KV cache");
+    auto kern = rvua::paged_decode_fp8_items_kernel<HD, GT, OutT>;
+    using C = rvua::ItemCfg<HD>;
+    static RvDeviceOnce smem_once;  // per kernel instantiation and device
+    if (rv_allow_smem(smem_once, kern, C::smem_bytes(C::MOST_UNITS)))
+        return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
+    const int ring = g_ring_units.load();
+    const long long ctas = (long long)p.kv_heads * p.max_chunks * p.batch;
+    int units = ring > 0 ? ring : rvua::pick_units<C>(ctas);
+    if (units < C::MIN_UNITS) units = C::MIN_UNITS;
+    if (units > C::MOST_UNITS) units = C::MOST_UNITS;
+    const int ordered = p.window_size_left < 0 && p.batch > 1 && p.batch <= rvua::ORDER_MAX;
+    rv_launch(kern, dim3(p.kv_heads, p.max_chunks, p.batch), dim3(rvua::THREADS), (size_t)C::smem_bytes(units), s, dim3(1, 1, 1),
+              mk, mv, mq, p, units, ordered);
+    return rv_launched("paged_decode_fp8 (tcgen05)");
+}
+
+template <int HD, int GT, typename OutT>
 int launch_umma(const rvattn::Params& p, cudaStream_t s) {
+    if (rvua::prefer_items<HD, GT>(p)) return launch_items<HD, GT, OutT>(p, s);
     return p.cluster_combine ? launch_umma_form<HD, GT, OutT, true>(p, s) : launch_umma_form<HD, GT, OutT, false>(p, s);
 }
 

@@ -871,8 +871,7 @@ inline bool supports_wide(const Params& p, int head_dim) { return head_dim == 51
 // deep one lets a CTA run further ahead of its softmax.  The choice minimises
 // ceil(CTAs / resident CTAs) x (relative time of one wave), with the per-wave weights measured on the
 // decode shapes (batch 8 / 32 / 128, contexts 576 to 4096).
-template <int HD> inline int pick_units(long long ctas, int extra_bytes = 0) {
-    using C = Cfg<HD>;
+template <typename C> inline int pick_units(long long ctas, int extra_bytes = 0) {
     struct Cand {
         int units;
         double wave;

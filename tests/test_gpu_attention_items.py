@@ -1,0 +1,68 @@
+"""Grids of more blocks than are resident at once: the attention kernel whose CTAs take over blocks that have not started."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from tests import datagen  # noqa: E402
+from tests.test_gpu_attention import assert_close, dev, run_oracle, run_ours  # noqa: E402
+
+# tile and page edges, the shortest, several tiles, and ones that fill nothing
+LENGTHS = [1, 127, 128, 129, 16, 300, 40, 256, 5, 520]
+
+
+def build(orc, batch, H_, KVH, HD, bs, window, seed):
+    ctxs = [LENGTHS[i % len(LENGTHS)] + (i // 40) * 3 for i in range(batch)]
+    mb = None if window < 0 else (window + bs) // bs + 1
+    c = datagen.attention_case(orc, batch, H_, KVH, HD, bs, ctxs, seed=seed, window=window, max_blocks=mb)
+    return c
+
+
+def check_status():
+    from rvllm_b200 import _lib
+    st = ctypes.c_int(0)
+    assert _lib.lib().rvllm_paged_decode_tc_status(ctypes.byref(st), 1) == 0 and st.value == 0
+
+
+# head_dim and query heads per KV head decide how many blocks are resident (740 down to 296); more than 256 sequences are not sorted
+@pytest.mark.parametrize("H_,KVH,HD,bs,batch,window", [(8, 4, 128, 16, 190, -1), (4, 4, 128, 32, 300, -1), (16, 4, 128, 8, 120, 255),
+                                                       (32, 4, 128, 16, 80, -1), (8, 4, 256, 16, 150, -1), (16, 2, 256, 128, 160, -1),
+                                                       (8, 4, 256, 16, 260, 63), (4, 2, 512, 16, 150, -1)])
+def test_more_blocks_than_resident(orc, H_, KVH, HD, bs, batch, window):
+    from rvllm_b200 import _lib
+    _lib.lib().rvllm_paged_decode_tune(0, 0, 0)
+    c = build(orc, batch, H_, KVH, HD, bs, window, seed=61 + HD + batch)
+    ctx = c["ctx"].copy()
+    ctx[3::37] = 0
+    ctx[5::41] = -2
+    if window < 0:
+        ctx[7::43] = c["max_blocks"] * bs + 1  # longer than the table: NaN
+        c["tables"][11, 0] = c["num_blocks"]   # outside the cache: NaN
+    c["ctx"] = ctx
+    assert_close(run_ours(c), run_oracle(orc, c, precise=True))
+    check_status()
+
+
+# the form that leaves partials for the quantising pass: the bytes of the plain call's output, quantised
+@pytest.mark.parametrize("HD,batch", [(128, 190), (256, 120)])
+def test_partials_for_the_quantiser(orc, HD, batch):
+    from rvllm_b200 import _lib, F16
+    from rvllm_b200.attention import PagedDecodeFp8Launcher, PagedDecodeParams
+    from rvllm_b200.launchers import QuantizeFp8PerTokenLaunch
+    _lib.lib().rvllm_paged_decode_tune(0, 0, 0)
+    c = build(orc, batch, 8, 4, HD, 16, -1, seed=71 + HD)
+    out = dev(run_ours(c)).half()
+    p = PagedDecodeParams(batch, 8, 4, HD, 16, c["max_blocks"], c["num_blocks"], c.get("scale", 1.0 / np.sqrt(HD)), -1)
+    la = PagedDecodeFp8Launcher(p)
+    ws = torch.empty(max(la.quant_workspace_bytes(), 256), dtype=torch.uint8, device="cuda")
+    got, gots = torch.empty((batch, 8 * HD), dtype=torch.uint8, device="cuda"), torch.empty(batch, device="cuda")
+    la.launch_quant(dev(c["q"]), dev(c["k"]), dev(c["v"]), got, gots, F16, dev(c["tables"]), dev(c["ctx"]), ws,
+                    k_scale_cache=dev(c["ks"]), v_scale_cache=dev(c["vs"]), q_scale_cache=dev(c["qs"]))
+    want, wants = torch.empty_like(got), torch.empty_like(gots)
+    QuantizeFp8PerTokenLaunch(batch, 8 * HD).launch(want, wants, out.reshape(batch, -1))
+    torch.cuda.synchronize()
+    assert torch.equal(gots, wants) and torch.equal(got, want)
+    check_status()
