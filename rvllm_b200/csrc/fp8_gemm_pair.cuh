@@ -614,15 +614,18 @@ inline int pair_recv_slots(int V, int S) {
     }
     return most;
 }
-// Tile width and split-K factor of a shape: the cheapest of the candidates under a cost model in microseconds, fitted to a
-// sweep of 16 weight shapes (512 x 512 to 43008 x 5376) and 20 batch sizes (4 to 2048): on it the choice is 1.4 % off the
-// best candidate on average, 23 % at worst (launches of 6 us).
+// Tile width and split-K factor of a shape: the cheapest of the candidates under a cost model in microseconds.  All widths are
+// candidates: weights of few rows fill the chip only with narrow batch tiles (512 x 512 at 1400 rows: 12 tiles of 256 columns 10.8
+// us, 88 of 32 5.7), and a short K spends its time in the epilogue between two tiles.  Over 16 weight shapes (512 x 512 to
+// 43008 x 5376) and 9 batch sizes (48 to 2048) the choice is 2 % off the best width on average, 15 % at worst.
 inline PairPlan pair_plan(int M, int N, int K, int ranges) {
-    const int nw = (N + 255) / 256, kblocks = (K + BK - 1) / BK, nb0 = (M + 255) / 256;
+    const int nw = (N + 255) / 256, kblocks = (K + BK - 1) / BK;
     PairPlan best = {};
     double best_cost = 0.0;
-    for (int want = nb0; want <= nb0 + 4; want++) {
-        const int bn = ((M + want - 1) / want + 31) / 32 * 32;
+    // (many rows run at the power cap, where a narrower tile, which moves more and pads more, must be worth it: 43008 x 5376 at 1000
+    // rows 158 us with 256 columns, 175 with 160, which the model puts 1 % ahead)
+    const double worth = M > 512 ? 0.96 : 1.0;
+    for (int bn = M > 224 ? 256 : (M + 31) / 32 * 32; bn >= 32; bn -= 32) {
         const int nb = (M + bn - 1) / bn, tiles = nw * nb;
         for (int S = 1; S <= 3; S++) {
             // (clusters of 4 and 6 CTAs: 32 and 21 of them were resident at once where measured, 35 and 25 were not)
@@ -634,12 +637,12 @@ inline PairPlan pair_plan(int M, int N, int K, int ranges) {
             const int sets = 2 * npart * bn <= 512 ? 2 : 1;
             const int waves = S > 1 ? 1 : (tiles + PAIRS - 1) / PAIRS;
             const double per_kb = fmax(1.464e-3 * bn, 0.178 + 2.4e-4 * bn);  // tensor pipe / issue and feed of 128 bytes of K
-            const double epi = 7e-3 * bn + 2e-3 * bn * (npart - 1);
+            const double epi = 1.6 + 0.019 * bn + 2e-3 * bn * (npart - 1);  // an epilogue between two tiles
             double us = ((kblocks + S - 1) / S) * per_kb;
-            us = waves * (sets == 2 ? fmax(us, epi) : us + (waves > 1 ? epi : 0.0));
+            us += (waves - 1) * (sets == 2 ? fmax(us, epi) : us + epi);  // (the last one's is in the constants below)
             us = fmax(us, (double)N * K / 7.88e6);  // the weights' stream
             us += 1.8 + 0.021 * bn + 2e-3 * bn * (npart - 1) + (S > 1 ? 0.86 + 8.2e-3 * bn * (1 + 0.5 * (npart - 1)) : 0.0);
-            if (best.bn == 0 || us < best_cost) {
+            if (best.bn == 0 || us < worth * best_cost) {
                 best = {bn, nb, tiles, S, V, npart, sets};
                 best_cost = us;
             }
