@@ -767,7 +767,9 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
 }
 
 // ---- host side -------------------------------------------------------------------------
-// Which launches take this kernel: one chunk per sequence and more blocks than the one-item kernel keeps resident at once.  Measured,
+// Which launches take this kernel: one chunk per sequence and more blocks than the one-item kernel keeps resident at once.
+// (With a window the lengths are mostly equal, there is nothing to reorder, and it takes two waves: 64 sequences that fill a window of
+// 1024, 52.8 / 53.5 us.)  Measured,
 // us, one-item kernel (in the callers' order) / this one, 32 query and 16 KV heads: 128 sequences of 48 tokens, head_dim 128, 22.5 /
 // 14.8, head_dim 256 41.0 / 24.2; 128 of 516 63.6 / 58.5; 32 of 600, head_dim 256, 36.3 / 33.8; 64 of 512 to 32768, head_dim 256, 1417
 // / 1291; 64 of 16 to 4000, 64 / 8 heads, 88.3 / 66.8; 64 of 1024 49.8 / 49.8; of 2000 91.4 / 92.5.  A grid that is resident at once
@@ -779,7 +781,8 @@ template <int HD, int GT> inline bool prefer_items(const Params& p) {
     if (p.max_chunks > 1 || p.amax_out) return false;
     const long long ctas = (long long)p.kv_heads * p.max_chunks * p.batch;
     const int fit = (228 * 1024) / (Cfg<HD>::smem_bytes(pick_units<Cfg<HD>>(ctas)) + 1024), regs = ctas_per_sm<HD, GT>();
-    return ctas > (long long)(HD != 512 && fit > regs ? regs : fit) * rv::SMS;
+    const long long resident = (long long)(HD != 512 && fit > regs ? regs : fit) * rv::SMS;
+    return ctas > (p.window_size_left < 0 ? resident : 2 * resident);
 }
 
 }  // namespace rvua

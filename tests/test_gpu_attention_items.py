@@ -28,7 +28,7 @@ def check_status():
 
 
 # head_dim and query heads per KV head decide how many blocks are resident (740 down to 296); more than 256 sequences are not sorted
-@pytest.mark.parametrize("H_,KVH,HD,bs,batch,window", [(8, 4, 128, 16, 190, -1), (4, 4, 128, 32, 300, -1), (16, 4, 128, 8, 120, 255),
+@pytest.mark.parametrize("H_,KVH,HD,bs,batch,window", [(8, 4, 128, 16, 190, -1), (4, 4, 128, 32, 300, -1), (16, 4, 128, 8, 240, 255),
                                                        (32, 4, 128, 16, 80, -1), (8, 4, 256, 16, 150, -1), (16, 2, 256, 128, 160, -1),
                                                        (8, 4, 256, 16, 260, 63), (4, 2, 512, 16, 150, -1)])
 def test_more_blocks_than_resident(orc, H_, KVH, HD, bs, batch, window):
