@@ -63,7 +63,7 @@ class PagedDecodeFp8Launcher:
                                              q_scale_cache, q_descale, k_descale, v_descale, p.scale, p.num_seqs,
                                              p.num_heads, p.num_kv_heads, p.head_dim, p.block_size,
                                              p.max_blocks_per_seq, p.num_blocks_total, p.window_size_left,
-                                             _lib.current_stream() if stream is None else stream)
+                                             _lib.launch_stream() if stream is None else stream)
         if rc:
             p.validate()  # (the same checks the call has just made: names the parameter set that failed)
             check(rc, "paged_decode_fp8")
@@ -82,7 +82,7 @@ class PagedDecodeFp8Launcher:
                                                    q_scale_cache, q_descale, k_descale, v_descale, p.scale, p.num_seqs,
                                                    p.num_heads, p.num_kv_heads, p.head_dim, p.block_size,
                                                    p.max_blocks_per_seq, p.num_blocks_total, p.window_size_left,
-                                                   _lib.current_stream() if stream is None else stream)
+                                                   _lib.launch_stream() if stream is None else stream)
         if rc:
             p.validate()
             check(rc, "paged_decode_fp8_quant")

@@ -998,15 +998,23 @@ inline bool cached_map(CUtensorMap* out, const void* base, int rows, int K, int 
     static std::mutex mu;
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
     MapKey key{base, rows, K, box};
+    static thread_local RvRecent<MapKey, CUtensorMap> recent;
+    const size_t hash = MapKeyHash()(key);
+    if (const CUtensorMap* m = recent.find(key, hash)) {
+        *out = *m;
+        return true;
+    }
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it != cache.end()) {
         *out = it->second;
+        recent.put(key, hash, *out);
         return true;
     }
     if (!make_map(out, base, rows, K, box)) return false;
     if (cache.size() > 4096) cache.clear();
     cache.emplace(key, *out);
+    recent.put(key, hash, *out);
     return true;
 }
 

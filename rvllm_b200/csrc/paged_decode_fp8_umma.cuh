@@ -835,10 +835,17 @@ inline bool cache_map(CUtensorMap* out, const void* base, long long slots, int k
     static std::mutex mu;
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
     MapKey key{base, slots, kv_heads, hd, bs};
+    static thread_local RvRecent<MapKey, CUtensorMap> recent;
+    const size_t hash = MapKeyHash()(key);
+    if (const CUtensorMap* m = recent.find(key, hash)) {
+        *out = *m;
+        return true;
+    }
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it != cache.end()) {
         *out = it->second;
+        recent.put(key, hash, *out);
         return true;
     }
     auto fn = encode_fn();
@@ -853,6 +860,7 @@ inline bool cache_map(CUtensorMap* out, const void* base, long long slots, int k
         return false;
     if (cache.size() > 4096) cache.clear();
     cache.emplace(key, *out);
+    recent.put(key, hash, *out);
     return true;
 }
 

@@ -23,7 +23,7 @@ def fp8_gemm_channelscale(out, a_fp8, w_fp8, a_scale, w_scale, residual=None, im
                           stream=None) -> None:
     """out[M, N] = cast(a_scale[m] * (w_scale[n] * A[M, K] . W[N, K]^T) (+ residual))."""
     if stream is None:
-        stream = _lib.current_stream()
+        stream = _lib.launch_stream()
     rc = native().gemm(out, a_fp8, w_fp8, a_scale, w_scale, residual, impl, workspace, stream)
     if rc is not None:
         if rc:
@@ -48,7 +48,7 @@ def fp8_gemm_gateup_act_quant(out_fp8, out_scale, a_fp8, w_fp8, a_scale, w_scale
     I = w_fp8.shape[0] // 2
     rc = native().rvllm_fp8_gemm_gateup_act_quant(out_fp8, out_scale, a_fp8, w_fp8, a_scale, w_scale, M, I, K, act, dtype, impl,
                                                   workspace, workspace.nbytes,
-                                                  _lib.current_stream() if stream is None else stream)
+                                                  _lib.launch_stream() if stream is None else stream)
     if rc:
         check(rc, "fp8_gemm_gateup_act_quant")
 

@@ -34,7 +34,7 @@ def _dtype_code(t) -> int:
 
 
 def _stream(stream):
-    return _lib.current_stream() if stream is None else stream
+    return _lib.launch_stream() if stream is None else stream
 
 
 def _refused(launch, rc, what):
