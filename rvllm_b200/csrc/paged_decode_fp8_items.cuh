@@ -32,8 +32,8 @@ __device__ __forceinline__ int uniform(int v) { return (int)__reduce_or_sync(0xf
 
 // ---- sequences by falling attended length ------------------------------------------------------------------------------
 // Blocks start in grid order, the batch outermost.  Where the grid takes more than one wave, that order is made the order of
-// falling length, so that the longest sequences do not start last (64 sequences of 512 to 32768 tokens, head_dim 256: 1490 us in
-// the callers' order).  Nothing is kept: every CTA sorts the batch, by counting, in its first microsecond.
+// falling length, so that the longest sequences do not start last (64 sequences of 512 to 32768 tokens, head_dim 256: 1614 us in the
+// callers' order, 1290 in this one).  Nothing is kept: every CTA sorts the batch, by counting, in its first microsecond.
 constexpr int ORDER_MAX = 256;  // sequences it is done for (a thread or two each)
 // Keys that fall with the attended length, then with the sequence's number.  True if this thread saw two lengths.
 __device__ __forceinline__ bool order_keys(const Params& p, int* key, int tid) {
@@ -257,8 +257,7 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
         const bool one = rv::elect_one();
         auto wait_one = [&](uint64_t* bar, uint32_t parity, int site) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, site)) != 0; };
         while (alive) {
-            // (uniform(): the compiler then knows them to be the same in all lanes, without which it issues each TMA
-            // instruction out of a loop over the lanes' values, 200 cycles instead of 70)
+            // (one value in all lanes: the loads below are issued by one elected lane from uniform registers)
             Item it;
             x = uniform(x);
             y = uniform(y);
@@ -768,15 +767,15 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
 
 // ---- host side -------------------------------------------------------------------------
 // Which launches take this kernel: one chunk per sequence and more blocks than the one-item kernel keeps resident at once.
-// (With a window the lengths are mostly equal, there is nothing to reorder, and it takes two waves: 64 sequences that fill a window of
-// 1024, 52.8 / 53.5 us.)  Measured,
-// us, one-item kernel (in the callers' order) / this one, 32 query and 16 KV heads: 128 sequences of 48 tokens, head_dim 128, 22.5 /
-// 14.8, head_dim 256 41.0 / 24.2; 128 of 516 63.6 / 58.5; 32 of 600, head_dim 256, 36.3 / 33.8; 64 of 512 to 32768, head_dim 256, 1417
-// / 1291; 64 of 16 to 4000, 64 / 8 heads, 88.3 / 66.8; 64 of 1024 49.8 / 49.8; of 2000 91.4 / 92.5.  A grid that is resident at once
-// gains nothing and pays for the records and claims (its page loads, whose operands are per item, take 140 cycles against 70): 33
-// sequences of 22 to 411 tokens 12.0 / 13.3, 19 of 300 to 4000, head_dim 256, 73.7 / 88.5, 12 at head_dim 512 81.7 / 109.8.  So do
-// grids whose blocks are chunks that short sequences leave empty, and the form that leaves maxima for the O projection, which is part
-// of a chain of dependent launches (32 rows, a 12-layer stack: 1465 / 1476 us per step).
+// With a window the lengths are mostly equal, there is nothing to reorder, and it takes two waves (64 sequences that fill a window of
+// 1024: 52.8 / 53.5 us).  Measured, us, one-item kernel (in the callers' order) / this one, 32 query and 16 KV heads unless stated: 128
+// sequences of 48 tokens, head_dim 128, 22.5 / 14.8, head_dim 256 41.0 / 24.2; 128 of 516 63.6 / 58.5; 32 of 600, head_dim 256, 36.3 /
+// 33.8; 64 of 512 to 32768, head_dim 256, 1417 / 1291; 64 of 16 to 4000, 64 / 8 heads, 88.3 / 66.8; 64 of 2000 91.4 / 92.5.
+// A grid that is resident at once gains nothing and pays for the records and claims (its page loads, whose operands are per item, take
+// 140 cycles against 70): 33 sequences of 22 to 411 tokens 12.0 / 13.3, 19 of 300 to 4000, head_dim 256, 73.7 / 88.5, 12 at head_dim 512
+// 81.7 / 109.8.  So do grids whose blocks are chunks that short sequences leave empty (15 sequences of up to 56 tokens, a whole layer
+// 126.5 / 132.8), and the form that leaves maxima for the O projection, which is part of a chain of dependent launches (32 rows, a
+// 12-layer stack: 1465 / 1476 us per step).
 template <int HD, int GT> inline bool prefer_items(const Params& p) {
     if (p.max_chunks > 1 || p.amax_out) return false;
     const long long ctas = (long long)p.kv_heads * p.max_chunks * p.batch;
