@@ -297,6 +297,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     auto rope_group = [&](int b, int g, int tile, int m_base, float ws, const float* as, const float* v) {
         if constexpr (ROPE) {
             const RopeKv& rk = p.rope;
+            // An odd number of heads leaves the last pair's second CTA without one (the whole CTA returns: nobody waits below).
+            if (tile >= rk.heads + 2 * rk.kv_heads) return;
             const int kind = tile < rk.heads ? 0 : (tile < rk.heads + rk.kv_heads ? 1 : 2);
             const int head = kind == 0 ? tile : (kind == 1 ? tile - rk.heads : tile - rk.heads - rk.kv_heads);
             float* stage = reinterpret_cast<float*>(header + PAIR_HEADER) + (size_t)((wg * 2 + (rope_use++ & 1)) * 16) * TILE_W;

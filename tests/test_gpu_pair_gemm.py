@@ -115,3 +115,41 @@ def test_pair_qkv_rope_at_odd_addresses(M, off):
 
     want, got = call(()), call(off)
     assert all(torch.equal(want[k], got[k]) for k in want)
+
+
+# an odd number of heads: the last CTA pair's second half holds no head, and must store none (consecutive slots, so that a
+# row too many would land on the next token's first head, and guards behind both caches and their scales)
+@pytest.mark.parametrize("M", [33, 128])
+@pytest.mark.parametrize("heads,kv_heads", [(7, 1), (5, 5), (3, 3)])
+def test_pair_qkv_rope_odd_heads(heads, kv_heads, M):
+    from rvllm_b200 import gemm, launchers
+    HD, K, guard = 128, 1024, 4 * kv_heads
+    N, rows = (heads + 2 * kv_heads) * HD, M * kv_heads
+    g = torch.Generator(device="cuda")
+    g.manual_seed(heads + M)
+    codes = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    a, w = codes(M, K), codes(N, K)
+    a_s, w_s = torch.rand(M, generator=g, device="cuda") * 0.1, torch.rand(N, generator=g, device="cuda") * 0.1
+    ang = torch.rand((M, HD // 2), generator=g, device="cuda") * 6.28
+    cos, sin = ang.cos().bfloat16(), ang.sin().bfloat16()
+    pos = torch.arange(M, dtype=torch.int32, device="cuda")
+    slot = pos.clone()
+
+    def buffers():
+        out = {k: torch.full((n + guard, HD), 0xAB, dtype=torch.uint8, device="cuda")
+               for k, n in dict(q8=M * heads, kc=rows, vc=rows).items()}
+        out.update({k: torch.full((n + guard,), -7.0, device="cuda") for k, n in dict(qs=M * heads, ks=rows, vs=rows).items()})
+        return out
+
+    def views(o):
+        return (o["q8"][:M * heads].view(M, heads, HD), o["qs"][:M * heads], o["kc"][:rows].view(M, kv_heads, HD),
+                o["vc"][:rows].view(M, kv_heads, HD), o["ks"][:rows], o["vs"][:rows])
+
+    got, want = buffers(), buffers()
+    assert launchers.qkv_rope_fp8kv(a, w, a_s, w_s, heads, kv_heads, HD, cos, sin, pos, slot, *views(got))
+    qkv = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    gemm.fp8_gemm_channelscale(qkv, a, w, a_s, w_s)
+    launchers.rope_fp8kv(qkv, heads, kv_heads, HD, HD, cos, sin, pos, slot, *views(want))
+    torch.cuda.synchronize()
+    assert gemm.tc_status() == 0
+    assert all(torch.equal(want[k], got[k]) for k in want)
