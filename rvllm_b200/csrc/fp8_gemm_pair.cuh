@@ -215,6 +215,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             int s = 0, b = 0;
             uint32_t ph = 0, set_ph = 1;  // (the first pass over the sets does not wait)
             bool alive = true;
+            rv::pdl_wait();  // (the first product needs the activations: no bounded wait while the preceding kernel runs)
             for (int t = cluster_id; t < p.tiles && alive; t += clusters) {
                 alive = mbar_wait_cluster(acc_empty + b, set_ph, 22);
                 if (!alive) break;

@@ -394,6 +394,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint64_t desc0 = smem_desc_sw128(smem_u32(ring));
         int s = 0;
         uint32_t ph = 0;
+        rv::pdl_wait();  // (the first product needs the activations: no bounded wait while the preceding kernel runs)
         for (int i = 0; i < nkb; i++) {
             if (!mbar_wait(full + s, ph, 2)) break;
             if (lane == 0 && i == 0) trace_point(p.trace, 2);  // both operands of the first K block are in shared memory

@@ -286,6 +286,11 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
                 it.ntiles = -1;
             }
             const int sl = n & (ITEM_SLOTS - 1);
+            // (the other warps read their first record after the dependency wait: no bounded wait for them ahead of it)
+            if (n >= ITEM_SLOTS && !waited) {
+                rv::pdl_wait();
+                waited = true;
+            }
             if (n >= ITEM_SLOTS) alive = wait_one(item_free + sl, (uint32_t)(n / ITEM_SLOTS - 1) & 1u, 11);
             if (!alive) break;
             if (lane == 0) {
@@ -382,6 +387,7 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
         // waiting for.  (The second product from a softmax warp, behind a barrier of the four: 15.3 against 14.5 us at 128
         // sequences of 48 tokens, head_dim 128, and 34.3 against 29.3 at 256.)
         const bool one = rv::elect_one();
+        if (early) rv::pdl_wait();  // (the first product needs Q: the poll limit below must not run while the preceding kernel does)
         constexpr uint32_t idesc_qk = instr_desc(NQ, false), idesc_pv = instr_desc(NP, true);
         const uint64_t rdesc = desc_kmajor(smem_u32(ring)), vdesc0 = desc_mnmajor(smem_u32(ring)), pdesc = desc_kmajor(smem_u32(p_tile));
         // Each of the two streams waits for one barrier at a time and a round of the loop tests one barrier per stream: an event

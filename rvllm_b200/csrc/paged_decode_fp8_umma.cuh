@@ -379,10 +379,13 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
         if (ntiles > 0) {
             const int ppt = TOK / bs;  // pages per tile (<= 16)
             const bool one = rv::elect_one();
-            bool alive = true, bad_page = false;
+            bool alive = true, bad_page = false, waited = !early;
             int slot = 0, use = 0;  // ring position of the next unit (kept incrementally: NUNITS is a run-time value)
             for (int i = 0; i < ntiles && alive; i++) {
-                if (early && i == ntiles - 1) rv::pdl_wait();  // the newest token's K / V rows are in the last tile
+                if (early && i == ntiles - 1) {  // the newest token's K / V rows are in the last tile
+                    rv::pdl_wait();
+                    waited = true;
+                }
                 const int tok_tile = tile0 + i * TOK;
                 // pages of the tile that hold attended tokens; the rest are not fetched (their rows of the
                 // unit keep stale bytes: masked in the scores, zeroed by the softmax warps for the V panels)
@@ -391,7 +394,12 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                 if (lane < np) z = phys_of(tok_tile + lane * bs, bad_page) * bs;
 #pragma unroll 1
                 for (int u = 0; u < UPT && alive; u++) {
-                    if (use > 0) alive = __all_sync(0xffffffffu, mbar_wait(empty + slot, (uint32_t)(use - 1) & 1u, 1)) != 0;
+                    if (use > 0) {
+                        // (a unit is freed by products, which need Q: no bounded wait for them while the preceding kernel runs)
+                        if (!waited) rv::pdl_wait();
+                        waited = true;
+                        alive = __all_sync(0xffffffffu, mbar_wait(empty + slot, (uint32_t)(use - 1) & 1u, 1)) != 0;
+                    }
                     if (!alive) break;
                     if (one) mbar_expect_tx(full + slot, (uint32_t)(np * bs * PANEL));
                     load_pages(ring + (size_t)slot * UNIT, bs * PANEL, u < HALVES ? &map_k : &map_v, (u % HALVES) * PANEL, kvh, z, np, one,

@@ -52,3 +52,36 @@ def test_read_only_loads_touch_weights_only():
             elif not READ_ONLY.search(arg) or re.search(r"\bp\.", arg):
                 bad.append(f"{name}: {arg}")
     assert not bad, bad
+
+
+# A bounded wait that depends on what the preceding kernel writes may only start once that kernel is complete: its limit counts
+# polls, and would otherwise run while the predecessor does.  Per wait: the file, the text that begins the warp role it is in,
+# the wait.  (The others of these kernels' waits follow one of these, or griddepcontrol.wait of the whole block.)
+BOUNDED = [
+    ("paged_decode_fp8_items.cuh", "if (warp == 0) {", "alive = wait_one(item_free"),
+    ("paged_decode_fp8_items.cuh", "} else if (warp == 1) {", "test(item_full"),
+    ("paged_decode_fp8_items.cuh", "if (use > 0) {", "alive = alive && wait_one(empty"),
+    ("paged_decode_fp8_umma.cuh", "if (use > 0) {", "mbar_wait(empty + slot"),
+    ("paged_decode_fp8_umma.cuh", "if (warp != 0) {", "mbar_try_wait(s_free"),
+    ("fp8_gemm_pair.cuh", "if (warp == 0) {", "mbar_wait(empty + s"),
+    ("fp8_gemm_pair.cuh", "} else if (warp == 1) {", "mbar_wait_cluster(acc_empty"),
+    ("fp8_gemm_tc.cuh", "} else if (warp == 1) {", "mbar_wait(full + s, ph, 2)"),
+    ("fp8_layer_block.cuh", "if (stage == 0) {", "alive = slot_free(it + i);"),
+    ("fp8_layer_block.cuh", "} else if (warp == 1) {", "mbar_wait(acc_free"),
+]
+
+
+def test_bounded_waits_start_after_the_dependency_wait():
+    bad = []
+    for name, role, wait in BOUNDED:
+        text = dict(code())[name]
+        at, end = -1, -1
+        while True:  # the role's text: from its last beginning ahead of the wait up to the wait
+            begin = text.find(role, at + 1)
+            if begin < 0 or (end > 0 and begin > end):
+                break
+            at, end = begin, text.find(wait, begin)
+        assert at < 0 or end > 0, (name, wait)
+        if at < 0 or not re.search(r"pdl_wait\(\)|send_q\(\)", text[at:end]):
+            bad.append(f"{name}: {wait}")
+    assert not bad, bad

@@ -66,3 +66,41 @@ def test_partials_for_the_quantiser(orc, HD, batch):
     torch.cuda.synchronize()
     assert torch.equal(gots, wants) and torch.equal(got, want)
     check_status()
+
+
+# Lengths, tables and older cache rows read ahead of the kernel that writes Q: unequal lengths, a window, empty sequences first (in
+# the batch's order above 256 of them: whole runs of records before the first that waits for Q), no more than one tile
+@pytest.mark.parametrize("H_,KVH,HD,bs,batch,window,empty,cap", [(8, 4, 128, 16, 190, -1, 3, 9999), (16, 4, 128, 8, 240, 255, 2, 9999),
+                                                                 (8, 4, 256, 16, 150, -1, 0, 9999), (4, 4, 128, 32, 600, -1, 500, 9999),
+                                                                 (8, 4, 128, 16, 190, -1, 1, 100)])
+def test_reads_ahead_of_the_kernel_that_writes_q(orc, H_, KVH, HD, bs, batch, window, empty, cap):
+    from rvllm_b200 import _lib
+    from rvllm_b200.attention import PagedDecodeFp8Launcher, PagedDecodeParams
+    from rvllm_b200.launchers import QuantizeFp8PerTokenLaunch
+    L = _lib.lib()
+    L.rvllm_paged_decode_tune(0, 0, 0)
+    c = build(orc, batch, H_, KVH, HD, bs, window, seed=83 + HD + batch)
+    ctx = np.minimum(c["ctx"], cap).astype(np.int32)
+    ctx[:empty] = 0
+    p = PagedDecodeParams(batch, H_, KVH, HD, bs, c["max_blocks"], c["num_blocks"], 1.0 / np.sqrt(HD), window)
+    la, quant = PagedDecodeFp8Launcher(p), QuantizeFp8PerTokenLaunch(batch * H_, HD)
+    x = torch.randn((batch * H_, HD), generator=torch.Generator("cuda").manual_seed(batch), device="cuda").half()
+    k, v, ks, vs, tables = (dev(c[n]) for n in ("k", "v", "ks", "vs", "tables"))
+    lens = dev(ctx)
+    ws = torch.empty(max(p.workspace_bytes(), 16), dtype=torch.uint8, device="cuda")
+    outs = []
+    try:
+        for mode in (-1, 1):
+            L.rvllm_paged_decode_early_meta(mode)
+            q8, qs = torch.full((batch * H_, HD), 0x7F, dtype=torch.uint8, device="cuda"), torch.full((batch * H_,), float("nan"), device="cuda")
+            out = torch.full((batch, H_, HD), 123.0, dtype=torch.float16, device="cuda")
+            torch.cuda.synchronize()
+            quant.launch(q8, qs, x)
+            la.launch(q8, k, v, out, tables, lens, workspace=ws, k_scale_cache=ks, v_scale_cache=vs, q_scale_cache=qs)
+            torch.cuda.synchronize()
+            outs.append(out)
+    finally:
+        L.rvllm_paged_decode_early_meta(0)
+    assert torch.equal(outs[0], outs[1]) and not outs[0].isnan().any() and (outs[0] != 123.0).all()
+    assert (outs[0][:empty] == 0).all() and (outs[0][empty:].abs().amax(dim=(1, 2)) > 0).all()
+    check_status()
