@@ -49,7 +49,9 @@ typedef struct {
                             need (a ragged batch: rvllm_stack_seed_contexts); sliding layers always keep their
                             fixed ring of sliding_window tokens per sequence */
     int fused_block;     /* 1: where the shape allows (batch <= 32), everything between two attention calls is one
-                            launch (rvllm_fp8_layer_block); 0: always the stand-alone kernels.  Same bytes either way. */
+                            launch (rvllm_fp8_layer_block); 0: always the stand-alone kernels, which are faster below
+                            32 rows and above hidden 1024.  The same bytes where both cut K alike (the 31B layer);
+                            on small layers the block cuts K further, so that f32 sums round differently */
     int fused_argmax;    /* 1: the LM head keeps per-tile argmax winners and a merge picks the token
                             (rvllm_fp8_gemm_lm_head_argmax; no f32 logits are written, debug read 1 is refused);
                             0: f32 logits, then argmax.  Same tokens either way. */

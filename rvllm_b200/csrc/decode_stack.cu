@@ -431,13 +431,10 @@ int enqueue_step(rvllm_stack* s, int* launches, bool chained = false) {
         // multiple of 128, ffn <= 4 * hidden): O projection, RMSNorm + quant, gate|up, act*up + quant, down, and the
         // RMSNorm + quant that opens the next layer (or closes the stack).
         int blk = RVLLM_E_UNSUPPORTED;
-        // (Not in small stacks of few rows: below hidden 1024 the launches of the chain cost less than the block's five grid
-        // meetings, which its 32 CTAs do little between.  Eight layers, block / chain, us per step: 512 x 2048 at 1, 4 and 32 rows
-        // 280 / 226, 288 / 234, 319 / 337.  From 1024 on the caller's switch decides alone: 1024 x 2048 318 / 258, 321 / 252,
-        // 380 / 381, 2048 x 8192 436 / 305, 434 / 334, 503 / 444.  The block cuts the short K of such stacks further than the chain
-        // does, so that f32 sums round differently: ten layers of 512 x 2048 after 60 steps, 1 to 16 rows, the same tokens and a hidden
-        // state within 2.5e-3 of each other.)
-        if (c.gemm_impl != 1 && c.fused_block != 0 && s->blk_ws_bytes > 0 && !(H < 1024 && B <= 16)) {
+        // (The caller's switch decides.  What it decides between, eight layers, block / chain, us per step: 512 x 2048 at 1, 8, 16,
+        // 24, 31 and 32 rows 276 / 217, 280 / 246, 294 / 272, 332 / 319, 334 / 334, 320 / 336; 1024 x 2048 at 1, 8, 16, 24 and 32 320 /
+        // 259, 317 / 294, 333 / 318, 385 / 357, 384 / 385; 2048 x 8192 at 1, 16 and 32 424 / 297, 461 / 364, 494 / 439.)
+        if (c.gemm_impl != 1 && c.fused_block != 0 && s->blk_ws_bytes > 0) {
             const void* next_gamma = l + 1 < c.num_layers ? s->layers[l + 1].attn_norm_gamma : s->head.final_norm_gamma;
             blk = rvllm_fp8_layer_block(B, H, c.ffn, L.q_dim, c.act, c.dtype, c.rms_eps, have16 ? s->attn_out : nullptr,
                                         s->attn_amax, c.kv_heads, have16 ? nullptr : s->attn_fp8, s->attn_scale, W.o_w,

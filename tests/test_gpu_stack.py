@@ -185,6 +185,49 @@ def test_graph_eager_and_pdl_variants_agree_bitwise(orc):
         assert np.array_equal(resid, results[0][2])
 
 
+# the layer block in small stacks: the same bytes through the graph, eagerly and without programmatic launch, and the oracle's tokens
+@pytest.mark.parametrize("batch,hidden", [(8, 512), (24, 1024), (32, 512)])
+def test_layer_block_graph_eager_and_pdl_variants_agree_bitwise(batch, hidden):
+    from rvllm_b200 import _lib
+    from rvllm_b200.stack import DecodeStack, random_weights, tiny_shape
+    cfg = tiny_shape(batch, hidden=hidden, num_layers=3, global_every=3, sliding_window=24, prompt_len=8, max_context=64, max_steps=64,
+                     dtype=1, fused_block=1)
+    w = random_weights(cfg, seed=5)
+    prompt = np.random.default_rng(1).integers(0, cfg["vocab"], (batch, 8), dtype=np.int32)
+    L = _lib.lib()
+    results = []
+    try:
+        for pdl, eager in ((1, False), (1, True), (0, False)):
+            L.rvllm_b200_set_pdl(pdl)
+            st = DecodeStack(cfg, w)
+            assert st.launches_per_step() < 3 * 5 + 6  # five launches a layer, not ten
+            st.reset(prompt)
+            st.run(48, eager=eager)
+            st.sync()
+            results.append((st.tokens().copy(), st.debug_read(1).copy(), st.debug_read(0).copy()))
+            st.close()
+    finally:
+        L.rvllm_b200_set_pdl(1)
+    for toks, logits, resid in results[1:]:
+        assert np.array_equal(toks, results[0][0])
+        assert np.array_equal(logits.view(np.uint32), results[0][1].view(np.uint32))
+        assert np.array_equal(resid, results[0][2])
+    assert_waits_ok()
+
+
+def test_layer_block_greedy_decode_against_oracle_chain(orc):
+    from oracle.chain import greedy_parity
+    from rvllm_b200.stack import tiny_shape
+    steps, P = 256, 16
+    cfg = tiny_shape(batch=4, num_layers=2, global_every=2, sliding_window=32, prompt_len=P, max_context=P + steps,
+                     max_steps=P + steps, dtype=1, fused_block=1)
+    stack, w = make(cfg)
+    assert stack.launches_per_step() < 2 * 6 + 6
+    prompt = np.random.default_rng(0).integers(0, cfg["vocab"], (4, P), dtype=np.int32)
+    check_parity(greedy_parity(orc, stack, cfg, w, prompt, steps, LOGIT_TOL))
+    stack.close()
+
+
 def test_step_host_matches_device_feedback(orc):
     from rvllm_b200.stack import tiny_shape
     cfg = tiny_shape(batch=4, prompt_len=4, max_context=64, max_steps=64)
