@@ -39,6 +39,20 @@ bool current_stream(uintptr_t* out) {
     return !(*out == 0 && PyErr_Occurred());
 }
 
+// Torch's look-ups, at load.  CURRENT_STREAM is None with a torch that has none: the Python side then passes handles.  False: an error is set.
+bool find_current_stream() {
+    if (PyObject* c = PyImport_ImportModule("torch._C")) {
+        g_get_device = PyObject_GetAttrString(c, "_cuda_getDevice");
+        g_get_stream = g_get_device ? PyObject_GetAttrString(c, "_cuda_getCurrentRawStream") : nullptr;
+        Py_DECREF(c);
+        if (g_get_stream) g_current = PyObject_CallNoArgs((PyObject*)&PyBaseObject_Type);
+    }
+    if (!PyErr_Occurred()) return true;
+    if (!PyErr_ExceptionMatches(PyExc_ImportError) && !PyErr_ExceptionMatches(PyExc_AttributeError)) return false;
+    PyErr_Clear();
+    return true;
+}
+
 bool to_pointer(PyObject* o, uintptr_t* out) {
     if (o == Py_None) {
         *out = 0;
@@ -207,14 +221,10 @@ PyMODINIT_FUNC PyInit__native(void) {
         Py_DECREF(m);
         m = nullptr;
     }
-    // CURRENT_STREAM is None with a torch that has no such look-ups: the Python side then passes handles.
-    if (PyObject* c = m ? PyImport_ImportModule("torch._C") : nullptr) {
-        g_get_device = PyObject_GetAttrString(c, "_cuda_getDevice");
-        g_get_stream = g_get_device ? PyObject_GetAttrString(c, "_cuda_getCurrentRawStream") : nullptr;
-        Py_DECREF(c);
-        if (g_get_stream) g_current = PyObject_CallNoArgs((PyObject*)&PyBaseObject_Type);
+    if (m && !find_current_stream()) {
+        Py_DECREF(m);
+        m = nullptr;
     }
-    PyErr_Clear();
     if (m && PyObject_SetAttrString(m, "CURRENT_STREAM", g_current ? g_current : Py_None) != 0) {
         Py_DECREF(m);
         m = nullptr;

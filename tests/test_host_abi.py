@@ -156,6 +156,35 @@ def test_native_module_for_another_torch_is_a_hard_error(monkeypatch):
     assert e.value.code == _lib.E_ARTIFACT
 
 
+def test_native_module_names_what_stopped_its_loading():
+    """An allocation that fails while the module is set up is reported as such, whichever it is."""
+    import subprocess
+    import sys
+
+    pytest.importorskip("_testcapi")
+    child = """
+import importlib.util, sys
+import _testcapi, torch
+from rvllm_b200 import _lib
+path = _lib.native().__file__
+seen = []
+for n in range(120):
+    spec = importlib.util.spec_from_file_location("_native", path)
+    _testcapi.set_nomemory(n, n + 1)
+    try:
+        try:
+            spec.loader.create_module(spec)
+        finally:
+            _testcapi.remove_mem_hooks()
+        seen.append("loaded")
+    except BaseException as e:
+        seen.append(type(e).__name__)
+sys.exit(0 if set(seen) == {"MemoryError", "loaded"} else repr(seen))
+"""
+    r = subprocess.run([sys.executable, "-c", child], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_build_register_budget_check():
     """The build refuses a kernel that counts on three CTAs per SM when ptxas gave it more than 96 registers."""
     from rvllm_b200 import build
