@@ -137,7 +137,7 @@ int launch_umma_form(const rvattn::Params& p, cudaStream_t s) {
     // cluster-combine form: the chunks of a (sequence, KV head) are one cluster, the receive area sits behind the rest
     // (and counts when the ring depth is chosen: a third of the footprint at eight chunks)
     const size_t recv = p.cluster_combine ? (size_t)C::recv_bytes(p.max_chunks, p.heads / p.kv_heads) : 0;
-    int units = ring > 0 ? ring : rvua::pick_units<C>((long long)p.kv_heads * p.max_chunks * p.batch, (int)recv);
+    int units = ring > 0 ? ring : rvua::pick_units<C>((long long)p.kv_heads * p.max_chunks * p.batch, CL ? 32 : rvua::ctas_per_sm<HD, GT>(), (int)recv);
     if (units < C::MIN_UNITS) units = C::MIN_UNITS;
     if (units > C::MOST_UNITS) units = C::MOST_UNITS;
     while (units > C::MIN_UNITS && C::smem_bytes(units) + recv > (size_t)C::smem_bytes(C::MOST_UNITS)) units--;
@@ -162,7 +162,7 @@ int launch_items(const rvattn::Params& p, cudaStream_t s) {
         return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
     const int ring = g_ring_units.load();
     const long long ctas = (long long)p.kv_heads * p.max_chunks * p.batch;
-    int units = ring > 0 ? ring : rvua::pick_units<C>(ctas);
+    int units = ring > 0 ? ring : rvua::pick_units<C>(ctas, rvua::ctas_per_sm<HD, GT>());
     if (units < C::MIN_UNITS) units = C::MIN_UNITS;
     if (units > C::MOST_UNITS) units = C::MOST_UNITS;
     const int ordered = p.window_size_left < 0 && p.batch > 1 && p.batch <= rvua::ORDER_MAX;

@@ -146,11 +146,8 @@ template <int HD> struct ItemCfg : Cfg<HD> {
     }
 };
 
-// CTAs per SM that registers must allow (the ring's depth may allow fewer)
-template <int HD, int GT> constexpr int ctas_per_sm() { return HD == 512 ? 1 : GT > 4 ? 2 : GT > 2 ? 3 : HD == 128 ? 5 : 4; }
-
 template <int HD, int GT, typename OutT>
-__global__ void __launch_bounds__(THREADS, ctas_per_sm<HD, GT>())
+__global__ void __launch_bounds__(THREADS, HD == 512 ? 1 : ctas_per_sm<HD, GT>())
 paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                               const __grid_constant__ CUtensorMap map_q, Params p, int nunits, int ordered) {
     static_assert(HD == 128 || HD == 256 || HD == 512, "one, two or four 128-byte panels per cache row");
@@ -309,8 +306,8 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
                 if (lane == 0 && alive) {
                     mbar_expect_tx(q_full + qb, (uint32_t)(nh * HD));
                     for (int h = 0; h < HALVES; h++)
-                        tma_load_3d(q_tile + (qb * HALVES + h) * C::QP, &map_q, h * PANEL, 0,
-                                    it.b * p.heads + it.kvh * group, q_full + qb);
+                        tma_load_3d(smem_u32(q_tile + (qb * HALVES + h) * C::QP), &map_q, h * PANEL, 0, it.b * p.heads + it.kvh * group,
+                                    smem_u32(q_full + qb));
                 }
                 q_sent += alive ? 1 : 0;
                 __syncwarp();
@@ -346,8 +343,8 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
                     }
                     if (!alive) break;
                     if (one) mbar_expect_tx(full + slot, (uint32_t)(np * bs * PANEL));
-                    load_pages(ring + (size_t)slot * UNIT, bs * PANEL, u < HALVES ? &map_k : &map_v, (u % HALVES) * PANEL, it.kvh, zz, np, one,
-                               full + slot);
+                    load_pages(smem_u32(ring) + (uint32_t)(slot * UNIT), bs * PANEL, u < HALVES ? &map_k : &map_v, (u % HALVES) * PANEL, it.kvh,
+                               zz, np, one, smem_u32(full + slot));
                     if (++slot == NUNITS) {
                         slot = 0;
                         use++;
@@ -390,15 +387,16 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
         if (early) rv::pdl_wait();  // (the first product needs Q: the poll limit below must not run while the preceding kernel does)
         constexpr uint32_t idesc_qk = instr_desc(NQ, false), idesc_pv = instr_desc(NP, true);
         const uint64_t rdesc = desc_kmajor(smem_u32(ring)), vdesc0 = desc_mnmajor(smem_u32(ring)), pdesc = desc_kmajor(smem_u32(p_tile));
-        // Each of the two streams waits for one barrier at a time and a round of the loop tests one barrier per stream: an event
-        // is seen within some twenty instructions.
+        // A product is issued when everything that it reads is there: its barriers are tested in one go, by the elected lane, which
+        // a barrier that is not complete may suspend for a while.  (One barrier per stream and round, tested without suspension: a
+        // product was seen to be ready up to three rounds late, and the warp took issue slots from the others.  256 sequences of
+        // 4000 tokens, 64 / 8 heads, head_dim 128, three units: 548 us so, 518 this way.)
         int next_qk = 0, next_pv = 0;        // tiles, over all items
         int left = 0, item = 0, active = 0;  // score tiles left in the current item; records read; items with tiles begun
         uint32_t firsts = 0;                 // bit t & 7: tile t opens an item (next_qk runs at most three ahead of next_pv)
         uint32_t idle = 0;
         bool alive = true, ended = false, opens = false;
-        int q_stage = 0, v_stage = 0;  // what the stream waits for: see below
-        // ring position (slot, use count) of the next K / V panel, advanced incrementally: NUNITS is a run-time value
+        // ring position (slot, use count) of the first K panel of tile next_qk and of the first V panel of tile next_pv
         int q_slot = 0, q_use = 0, v_slot = HALVES % NUNITS, v_use = HALVES / NUNITS;
         auto step = [&](int& slot, int& use, int by) {
             slot += by;
@@ -416,13 +414,12 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
             const int tile = g / UPT;
             return g % UPT < HALVES ? tile < next_qk : tile < next_pv;
         };
-        auto test = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_test(bar, parity)); };
         while (alive && !(ended && next_pv == next_qk)) {
             bool did = false;
-            // ---- scores: a record, the TMEM buffer, Q, then panel after panel ----
+            // ---- scores: a record, then the TMEM buffer, Q and the K panels ----
             if (left == 0) {
                 const int sl = item & (ITEM_SLOTS - 1);
-                if (!ended && test(item_full + sl, (uint32_t)(item / ITEM_SLOTS) & 1u)) {
+                if (!ended && __all_sync(0xffffffffu, mbar_test(item_full + sl, (uint32_t)(item / ITEM_SLOTS) & 1u))) {
                     const int t = items[sl].ntiles;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(item_free + sl);
@@ -433,70 +430,76 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
                     active += t > 0 ? 1 : 0;
                     did = true;
                 }
-            } else if (q_stage == 0) {
-                if (next_qk < 2 || test(s_free + (next_qk & 1), (uint32_t)((next_qk >> 1) - 1) & 1u)) {
-                    q_stage = opens ? 1 : 2;
-                    did = true;
-                }
-            } else if (q_stage == 1) {
-                if (test(q_full + ((active - 1) & 1), (uint32_t)((active - 1) / 2) & 1u)) {
-                    q_stage = 2;
-                    did = true;
-                }
-            } else if (prev_consumed(next_qk * UPT + q_stage - 2) && test(full + q_slot, (uint32_t)q_use & 1u)) {
-                const int h = q_stage - 2, qb = (active - 1) & 1;
-                tc_fence_after();
-                if (one) {
-                    const uint64_t kdesc = rdesc + (uint64_t)((q_slot * UNIT) >> 4), qd = C::q_desc(smem_u32(q_tile), qb, h);
+            } else {
+                const int i = next_qk, qb = (active - 1) & 1;
+                bool ok = one && (i < 2 || mbar_try_wait(s_free + (i & 1), (uint32_t)((i >> 1) - 1) & 1u));
+                if (opens) ok = ok && mbar_try_wait(q_full + qb, (uint32_t)((active - 1) / 2) & 1u);
+                int slot[HALVES];
 #pragma unroll
-                    for (int k = 0; k < PANEL / 32; k++)
-                        umma_f8(tmem_base + (uint32_t)(next_qk & 1) * NQ, kdesc + (uint64_t)(2 * k), qd + (uint64_t)(2 * k), idesc_qk,
-                                (h > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(empty + q_slot);
+                for (int h = 0; h < HALVES; h++) {
+                    int sl = q_slot + h, us = q_use;
+                    if (sl >= NUNITS) {
+                        sl -= NUNITS;
+                        us++;
+                    }
+                    slot[h] = sl;
+                    ok = ok && prev_consumed(i * UPT + h) && mbar_try_wait(full + sl, (uint32_t)us & 1u);
                 }
-                step(q_slot, q_use, 1);
-                q_stage++;
-                if (h == HALVES - 1) {
+                if (__any_sync(0xffffffffu, ok)) {
+                    tc_fence_after();
                     left--;
                     if (one) {
-                        umma_commit(s_ready + (next_qk & 1));
+#pragma unroll
+                        for (int h = 0; h < HALVES; h++) {
+                            const uint64_t kdesc = rdesc + (uint64_t)((slot[h] * UNIT) >> 4), qd = C::q_desc(smem_u32(q_tile), qb, h);
+#pragma unroll
+                            for (int k = 0; k < PANEL / 32; k++)
+                                umma_f8(tmem_base + (uint32_t)(i & 1) * NQ, kdesc + (uint64_t)(2 * k), qd + (uint64_t)(2 * k), idesc_qk,
+                                        (h > 0 || k > 0) ? 1u : 0u);
+                            umma_commit(empty + slot[h]);
+                        }
+                        umma_commit(s_ready + (i & 1));
                         if (left == 0) umma_commit(q_free + qb);
                     }
-                    firsts = (firsts & ~(1u << (next_qk & 7))) | ((opens ? 1u : 0u) << (next_qk & 7));
+                    firsts = (firsts & ~(1u << (i & 7))) | ((opens ? 1u : 0u) << (i & 7));
                     opens = false;
                     next_qk++;
-                    step(q_slot, q_use, HALVES);
-                    q_stage = 0;
+                    step(q_slot, q_use, UPT);
+                    did = true;
                 }
-                did = true;
             }
-            // ---- second product: the P tile, then panel after panel ----
+            // ---- second product: the P tile and the V panels ----
             if (next_pv < next_qk) {
-                if (v_stage == 0) {
-                    if (test(p_ready, (uint32_t)next_pv & 1u)) {
-                        v_stage = 1;
-                        did = true;
+                const int i = next_pv;
+                bool ok = one && mbar_try_wait(p_ready, (uint32_t)i & 1u);
+                int slot[HALVES];
+#pragma unroll
+                for (int h = 0; h < HALVES; h++) {
+                    int sl = v_slot + h, us = v_use;
+                    if (sl >= NUNITS) {
+                        sl -= NUNITS;
+                        us++;
                     }
-                } else if (prev_consumed(next_pv * UPT + HALVES + v_stage - 1) && test(full + v_slot, (uint32_t)v_use & 1u)) {
-                    const int h = v_stage - 1;
+                    slot[h] = sl;
+                    ok = ok && prev_consumed(i * UPT + HALVES + h) && mbar_try_wait(full + sl, (uint32_t)us & 1u);
+                }
+                if (__any_sync(0xffffffffu, ok)) {
                     tc_fence_after();
                     if (one) {
-                        const uint64_t vdesc = vdesc0 + (uint64_t)((v_slot * UNIT) >> 4);
-                        const uint32_t add = (firsts >> (next_pv & 7)) & 1u ? 0u : 1u;
+                        const uint32_t add = (firsts >> (i & 7)) & 1u ? 0u : 1u;
 #pragma unroll
-                        for (int k = 0; k < TOK / 32; k++)  // 32 tokens (rows of 128 B) per MMA
-                            umma_f8(tmem_base + C::O_COL + (uint32_t)h * NP, vdesc + (uint64_t)((32 * PANEL * k) >> 4),
-                                    pdesc + (uint64_t)(2 * k), idesc_pv, k > 0 ? 1u : add);
-                        umma_commit(empty + v_slot);
-                        if (h == HALVES - 1) umma_commit(pv_done);
+                        for (int h = 0; h < HALVES; h++) {
+                            const uint64_t vdesc = vdesc0 + (uint64_t)((slot[h] * UNIT) >> 4);
+#pragma unroll
+                            for (int k = 0; k < TOK / 32; k++)
+                                umma_f8(tmem_base + C::O_COL + (uint32_t)h * NP, vdesc + (uint64_t)((32 * PANEL * k) >> 4),
+                                        pdesc + (uint64_t)(2 * k), idesc_pv, k > 0 ? 1u : add);
+                            umma_commit(empty + slot[h]);
+                        }
+                        umma_commit(pv_done);
                     }
-                    step(v_slot, v_use, 1);
-                    v_stage++;
-                    if (h == HALVES - 1) {
-                        next_pv++;
-                        step(v_slot, v_use, HALVES);
-                        v_stage = 0;
-                    }
+                    next_pv++;
+                    step(v_slot, v_use, UPT);
                     did = true;
                 }
             }
@@ -772,21 +775,28 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
 }
 
 // ---- host side -------------------------------------------------------------------------
-// Which launches take this kernel: one chunk per sequence and more blocks than the one-item kernel keeps resident at once.
-// With a window the lengths are mostly equal, there is nothing to reorder, and it takes two waves (64 sequences that fill a window of
-// 1024: 52.8 / 53.5 us).  Measured, us, one-item kernel (in the callers' order) / this one, 32 query and 16 KV heads unless stated: 128
-// sequences of 48 tokens, head_dim 128, 22.5 / 14.8, head_dim 256 41.0 / 24.2; 128 of 516 63.6 / 58.5; 32 of 600, head_dim 256, 36.3 /
-// 33.8; 64 of 512 to 32768, head_dim 256, 1417 / 1291; 64 of 16 to 4000, 64 / 8 heads, 88.3 / 66.8; 64 of 2000 91.4 / 92.5.
-// A grid that is resident at once gains nothing and pays for the records and claims (its page loads, whose operands are per item, take
-// 140 cycles against 70): 33 sequences of 22 to 411 tokens 12.0 / 13.3, 19 of 300 to 4000, head_dim 256, 73.7 / 88.5, 12 at head_dim 512
-// 81.7 / 109.8.  So do grids whose blocks are chunks that short sequences leave empty (15 sequences of up to 56 tokens, a whole layer
+// Which launches take this kernel: one chunk per sequence and more blocks than the one-item kernel keeps resident at once; with a
+// window, where nothing is reordered, from two waves on.  Lengths are not known here, and what it gives depends on them.  Measured,
+// us, one-item kernel (in the callers' order) / this one, 16-token pages:
+//   short       128 sequences of 48 tokens, 16 KV heads, head_dim 128 28.6 / 22.5; 256 of 516 121.5 / 114.9; 64 of 516, head_dim 512
+//               143 / 125
+//   unequal     64 of 500 to 16000, head_dim 128 397 / 381; 64 of 100 to 4000, 64 / 8 heads 105 / 72, head_dim 512 266 / 200, 32 / 16
+//               heads 360 / 335
+//   with a window of 1024: 256 of 16 to 400 tokens, head_dim 128 69.7 / 62.0; 256 of 100 to 4000, 64 / 8 heads, head_dim 256 229 / 215
+//   equal, long 64 of 2000, 16 KV heads, head_dim 128 102.7 / 106.6; 256 of 4000 631 / 670, with a window of 1024 182 / 187; 128 of 4000,
+//               64 / 8 heads, head_dim 256 390 / 382
+// So the cost is with equal long contexts at head_dim 128 and one or two query heads per KV head, which stream at the copy rate in
+// either kernel (3 to 6 %), and with short ones at head_dim 512 and more than four (40 of 48 tokens 33 / 37; 128 of 16 to 400 with a
+// window 92 / 101).
+// A grid that is resident at once gains nothing and pays for the records and claims: 33 sequences of 22 to 411 tokens 12.0 / 13.3.
+// So do grids whose blocks are chunks that short sequences leave empty (15 sequences of up to 56 tokens, a whole layer
 // 126.5 / 132.8), and the form that leaves maxima for the O projection, which is part of a chain of dependent launches (32 rows, a
 // 12-layer stack: 1465 / 1476 us per step).
 template <int HD, int GT> inline bool prefer_items(const Params& p) {
     if (p.max_chunks > 1 || p.amax_out) return false;
     const long long ctas = (long long)p.kv_heads * p.max_chunks * p.batch;
-    const int fit = (228 * 1024) / (Cfg<HD>::smem_bytes(pick_units<Cfg<HD>>(ctas)) + 1024), regs = ctas_per_sm<HD, GT>();
-    const long long resident = (long long)(HD != 512 && fit > regs ? regs : fit) * rv::SMS;
+    const int fit = (228 * 1024) / (Cfg<HD>::smem_bytes(pick_units<Cfg<HD>>(ctas, ctas_per_sm<HD, GT>())) + 1024);
+    const long long resident = (long long)(fit < ctas_per_sm<HD, GT>() ? fit : ctas_per_sm<HD, GT>()) * rv::SMS;
     return ctas > (p.window_size_left < 0 ? resident : 2 * resident);
 }
 

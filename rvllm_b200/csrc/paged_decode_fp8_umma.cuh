@@ -87,33 +87,39 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void bar_softmax() { asm volatile("bar.sync 1, 128;" ::: "memory"); }  // warps 2-5 only
 
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-        ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
         : "memory");
 }
-// The pages of one panel of a tile, page j's first slot in lane j.  One elected lane issues them out of a loop of the whole warp,
-// its operands in uniform registers: lanes that issue side by side are served one after another, 120 cycles each, against 70 here.
-// A tile of head_dim 256 in 16-token pages has 32 of these instructions, which made the producer the kernel's longest chain.
-__device__ __forceinline__ void load_pages(uint8_t* dst, int page_bytes, const CUtensorMap* map, int x, int head, int slots, int np, bool one,
-                                           uint64_t* bar) {
+// The pages of one panel of a tile, page j's first slot in lane j.  One elected lane issues them out of code of the whole warp, its
+// operands in uniform registers: lanes that issue side by side are served one after another, 120 cycles each.  A tile of head_dim 256
+// in 16-token pages has 32 of these instructions, which made the producer the kernel's longest chain.  Straight-line groups of
+// eight with 32-bit addresses: 45 cycles a page in both kernels, where groups of four with pointers took 46 in this one and 80 to 90 in
+// the items kernel, whose geometry is in per-thread registers.
+template <int N>
+__device__ __forceinline__ void load_group(uint32_t dst, int page_bytes, const CUtensorMap* map, int x, int head, int slots, int first, bool one,
+                                           uint32_t bar) {
+    int z[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) z[k] = __shfl_sync(0xffffffffu, slots, first + k);
+    if (one) {
+#pragma unroll
+        for (int k = 0; k < N; k++) tma_load_3d(dst + (uint32_t)(k * page_bytes), map, x, head, z[k], bar);
+    }
+}
+__device__ __forceinline__ void load_pages(uint32_t dst, int page_bytes, const CUtensorMap* map, int x, int head, int slots, int np, bool one,
+                                           uint32_t bar) {
     int j = 0;
 #pragma unroll 1
-    for (; j + 4 <= np; j += 4) {
-        int z[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) z[k] = __shfl_sync(0xffffffffu, slots, j + k);
-        if (one) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) tma_load_3d(dst + (size_t)(j + k) * page_bytes, map, x, head, z[k], bar);
-        }
+    for (; j + 8 <= np; j += 8) load_group<8>(dst + (uint32_t)(j * page_bytes), page_bytes, map, x, head, slots, j, one, bar);
+    if (j + 4 <= np) {
+        load_group<4>(dst + (uint32_t)(j * page_bytes), page_bytes, map, x, head, slots, j, one, bar);
+        j += 4;
     }
 #pragma unroll 1
-    for (; j < np; j++) {
-        const int z = __shfl_sync(0xffffffffu, slots, j);
-        if (one) tma_load_3d(dst + (size_t)j * page_bytes, map, x, head, z, bar);
-    }
+    for (; j < np; j++) load_group<1>(dst + (uint32_t)(j * page_bytes), page_bytes, map, x, head, slots, j, one, bar);
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t* holder, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)), "r"(cols)
@@ -402,8 +408,8 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
                     }
                     if (!alive) break;
                     if (one) mbar_expect_tx(full + slot, (uint32_t)(np * bs * PANEL));
-                    load_pages(ring + (size_t)slot * UNIT, bs * PANEL, u < HALVES ? &map_k : &map_v, (u % HALVES) * PANEL, kvh, z, np, one,
-                               full + slot);
+                    load_pages(smem_u32(ring) + (uint32_t)(slot * UNIT), bs * PANEL, u < HALVES ? &map_k : &map_v, (u % HALVES) * PANEL, kvh, z,
+                               np, one, smem_u32(full + slot));
                     if (++slot == NUNITS) {
                         slot = 0;
                         use++;
@@ -883,11 +889,15 @@ inline bool supports(const Params& p, int head_dim) { return (head_dim == 128 ||
 // tokens, 32 / 16 heads: 222 us on the mma.sync form, 89 here).
 inline bool supports_wide(const Params& p, int head_dim) { return head_dim == 512 && heads_and_pages_ok(p); }
 
+// CTAs per SM that registers allow (the ring's depth may allow fewer, and does at head_dim 512)
+template <int HD, int GT> constexpr int ctas_per_sm() { return HD == 512 ? 2 : GT > 4 ? 2 : GT > 2 ? 3 : HD == 128 ? 5 : 4; }
+
 // Ring depth.  A shallow ring lets more CTAs share an SM (the footprint is 8-10 KB + 16 KB per unit), a
 // deep one lets a CTA run further ahead of its softmax.  The choice minimises
 // ceil(CTAs / resident CTAs) x (relative time of one wave), with the per-wave weights measured on the
-// decode shapes (batch 8 / 32 / 128, contexts 576 to 4096).
-template <typename C> inline int pick_units(long long ctas, int extra_bytes = 0) {
+// decode shapes (batch 8 / 32 / 128, contexts 576 to 4096).  A ring made shallow for more CTAs than registers allow (`most` per SM) is only
+// shallow: it gets the deepest that keeps these (256 sequences of 4000 tokens, 64 / 8 heads, head_dim 128: three units 498 us, six 420).
+template <typename C> inline int pick_units(long long ctas, int most, int extra_bytes = 0) {
     struct Cand {
         int units;
         double wave;
@@ -897,16 +907,19 @@ template <typename C> inline int pick_units(long long ctas, int extra_bytes = 0)
     static const Cand c512[] = {{6, 1.15}, {12, 1.0}};
     const Cand* cand = C::HALVES == 1 ? c128 : C::HALVES == 2 ? c256 : c512;
     const int n = C::HALVES == 1 ? 4 : 2;
+    auto fit = [&](int units) { return (228 * 1024) / (C::smem_bytes(units) + extra_bytes + 1024); };
     int best = cand[0].units;
     double best_cost = 1e300;
     for (int i = 0; i < n; i++) {
-        const long long slots = ((228 * 1024) / (C::smem_bytes(cand[i].units) + extra_bytes + 1024)) * (long long)rv::SMS;
+        const long long slots = (long long)fit(cand[i].units) * rv::SMS;
         const double cost = (double)((ctas + slots - 1) / slots) * cand[i].wave;
         if (cost < best_cost) {
             best_cost = cost;
             best = cand[i].units;
         }
     }
+    for (int i = 0; i < n; i++)
+        if (cand[i].units > best && fit(best) > most && fit(cand[i].units) >= most) best = cand[i].units;
     return best;
 }
 
