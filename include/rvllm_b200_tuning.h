@@ -78,6 +78,9 @@ void rvllm_paged_decode_cluster_tune(int target_ctas, int min_chunk_tokens);
 /* Depth of the tcgen05 kernel's K/V ring in 16 KB units (2..8 for head_dim 128, 3..8 for 256);
  * 0 restores the automatic choice.  Tuning aid, process-wide. */
 void rvllm_paged_decode_ring(int units);
+/* Kernel of the calling thread's last decode-attention launch: the variants 1 to 4 of rvllm_paged_decode_tune, 5 for
+ * variant 4 with resident CTAs that take over blocks (unsplit grids of more than one wave), 0 before the first.  Diagnostic. */
+int rvllm_paged_decode_last_form(void);
 
 /* Timing aid: decode stacks created while a mask is set leave the marked launches out of every layer of their step
  * (1 attention-block RMSNorm, 2 QKV GEMM (+RoPE / KV write), 4 attention, 8 O projection, 16 MLP RMSNorm, 32 gate|up,

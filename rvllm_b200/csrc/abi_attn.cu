@@ -23,6 +23,7 @@ static thread_local int t_early_meta_once = 0;  // one-shot hint of the calling 
 static std::atomic<int> g_cluster_min_tokens{rvua::TOK};  // smallest chunk of the cluster-merged split-KV form
 static std::atomic<int> g_cluster_target{0};  // CTAs the cluster-merged form aims for, 0 = rvua::pick_cluster_chunks
 static std::atomic<int> g_ring_units{0};  // tcgen05 kernel: K/V ring depth in 16 KB units, 0 = automatic
+static thread_local int t_last_form = 0;  // kernel of the calling thread's last decode-attention launch
 static std::atomic<int> g_variant{0};  // 0 automatic (tcgen05 kernel where the shape allows, else 3, else 2), 1 FP32-pipe kernel,
                            // 2 mma.sync scores + FP32-pipe P.V, 3 both products on mma.sync, 4 tcgen05 / TMA
 
@@ -97,6 +98,7 @@ void rvllm_paged_decode_cluster_tune(int target_ctas, int min_chunk_tokens) {
 }
 
 void rvllm_paged_decode_ring(int units) { g_ring_units = units > 0 ? units : 0; }
+int rvllm_paged_decode_last_form(void) { return t_last_form; }
 
 int rvllm_paged_decode_tc_status(int* status, int reset) {
     if (!status) return rv_fail(RVLLM_E_INVALID, "null status pointer");
@@ -141,6 +143,7 @@ int launch_umma_form(const rvattn::Params& p, cudaStream_t s) {
     if (units < C::MIN_UNITS) units = C::MIN_UNITS;
     if (units > C::MOST_UNITS) units = C::MOST_UNITS;
     while (units > C::MIN_UNITS && C::smem_bytes(units) + recv > (size_t)C::smem_bytes(C::MOST_UNITS)) units--;
+    t_last_form = 4;
     rv_launch(kern, dim3(p.kv_heads, p.max_chunks, p.batch), dim3(rvua::THREADS), (size_t)C::smem_bytes(units) + recv, s,
               dim3(1, p.cluster_combine ? p.max_chunks : 1, 1), mk, mv, p, units);
     return rv_launched("paged_decode_fp8 (tcgen05)");
@@ -165,6 +168,7 @@ int launch_items(const rvattn::Params& p, cudaStream_t s) {
     int units = ring > 0 ? ring : rvua::pick_units<C>(ctas, rvua::ctas_per_sm<HD, GT>());
     if (units < C::MIN_UNITS) units = C::MIN_UNITS;
     if (units > C::MOST_UNITS) units = C::MOST_UNITS;
+    t_last_form = 5;
     const int ordered = p.window_size_left < 0 && p.batch > 1 && p.batch <= rvua::ORDER_MAX;
     rv_launch(kern, dim3(p.kv_heads, p.max_chunks, p.batch), dim3(rvua::THREADS), (size_t)C::smem_bytes(units), s, dim3(1, 1, 1),
               mk, mv, mq, p, units, ordered);
@@ -209,6 +213,7 @@ int launch_attn(const rvattn::Params& p, const QuantOut& qo, cudaStream_t s) {
         static RvDeviceOnce smem_once;  // per kernel instantiation and device
         if (smem > 48 * 1024 && rv_allow_smem(smem_once, kern, (int)smem))
             return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
+        t_last_form = 1;
         rv_launch(kern, grid, dim3(rvattn::THREADS), smem, s, dim3(1, 1, 1), p);
     } else if (g_variant != 2 && HD <= 256 &&
                (long long)p.num_blocks_total * p.block_size * p.kv_heads < (1ll << 31)) {
@@ -218,6 +223,7 @@ int launch_attn(const rvattn::Params& p, const QuantOut& qo, cudaStream_t s) {
             static RvDeviceOnce smem_once;  // per kernel instantiation and device
             if (smem > 48 * 1024 && rv_allow_smem(smem_once, kern, (int)smem))
                 return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
+            t_last_form = 3;
             rv_launch(kern, grid, dim3(rvattn::MMA_THREADS), smem, s, dim3(1, 1, 1), p);
         }
     } else {
@@ -226,6 +232,7 @@ int launch_attn(const rvattn::Params& p, const QuantOut& qo, cudaStream_t s) {
         static RvDeviceOnce smem_once;  // per kernel instantiation and device
         if (smem > 48 * 1024 && rv_allow_smem(smem_once, kern, (int)smem))
             return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
+        t_last_form = 2;
         rv_launch(kern, grid, dim3(rvattn::MMA_THREADS), smem, s, dim3(1, 1, 1), p);
     }
     int rc = rv_launched("paged_decode_fp8");

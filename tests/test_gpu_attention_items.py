@@ -42,7 +42,38 @@ def test_more_blocks_than_resident(orc, H_, KVH, HD, bs, batch, window):
         ctx[7::43] = c["max_blocks"] * bs + 1  # longer than the table: NaN
         c["tables"][11, 0] = c["num_blocks"]   # outside the cache: NaN
     c["ctx"] = ctx
-    assert_close(run_ours(c), run_oracle(orc, c, precise=True))
+    got = run_ours(c)
+    assert _lib.lib().rvllm_paged_decode_last_form() == 5
+    assert_close(got, run_oracle(orc, c, precise=True))
+    check_status()
+
+
+# the same sequences in batches whose grids are resident at once, unsplit, which the one-item kernel takes: the same bytes.  Up to
+# eight query heads per KV head, partly filled groups, every head_dim and page size, a window
+@pytest.mark.parametrize("H_,KVH,HD,bs,batch,window", [(4, 4, 128, 16, 300, -1), (12, 4, 128, 8, 190, -1), (32, 4, 128, 128, 90, -1),
+                                                       (20, 4, 128, 16, 160, 255), (8, 4, 256, 32, 190, -1), (28, 4, 256, 16, 100, -1),
+                                                       (8, 4, 256, 8, 260, 300), (4, 2, 512, 16, 150, -1), (16, 2, 512, 64, 170, -1)])
+def test_bytes_equal_to_the_one_item_kernels(orc, H_, KVH, HD, bs, batch, window):
+    from rvllm_b200 import _lib
+    L = _lib.lib()
+    L.rvllm_paged_decode_tune(0, 0, 0)
+    c = build(orc, batch, H_, KVH, HD, bs, window, seed=91 + HD + batch)
+    c["ctx"][4::29] = 0
+    got = run_ours(c)
+    assert L.rvllm_paged_decode_last_form() == 5
+    step = 64 // KVH
+    try:
+        L.rvllm_paged_decode_tune(1, 0, 0)  # (one CTA aimed for: nothing is split, through the workspace or in a cluster)
+        L.rvllm_paged_decode_cluster_combine(0)
+        for b in range(0, batch, step):
+            s = slice(b, min(b + step, batch))
+            part = dict(c, batch=s.stop - s.start, qs=c["qs"].reshape(batch, H_)[s], **{k: c[k][s] for k in ("ctx", "tables", "q")})
+            want = run_ours(part)
+            assert L.rvllm_paged_decode_last_form() == 4
+            assert got[s].tobytes() == want.tobytes(), b
+    finally:
+        L.rvllm_paged_decode_tune(0, 0, 0)
+        L.rvllm_paged_decode_cluster_combine(1)
     check_status()
 
 
@@ -61,6 +92,7 @@ def test_partials_for_the_quantiser(orc, HD, batch):
     got, gots = torch.empty((batch, 8 * HD), dtype=torch.uint8, device="cuda"), torch.empty(batch, device="cuda")
     la.launch_quant(dev(c["q"]), dev(c["k"]), dev(c["v"]), got, gots, F16, dev(c["tables"]), dev(c["ctx"]), ws,
                     k_scale_cache=dev(c["ks"]), v_scale_cache=dev(c["vs"]), q_scale_cache=dev(c["qs"]))
+    assert _lib.lib().rvllm_paged_decode_last_form() == 5
     want, wants = torch.empty_like(got), torch.empty_like(gots)
     QuantizeFp8PerTokenLaunch(batch, 8 * HD).launch(want, wants, out.reshape(batch, -1))
     torch.cuda.synchronize()
@@ -97,6 +129,7 @@ def test_reads_ahead_of_the_kernel_that_writes_q(orc, H_, KVH, HD, bs, batch, wi
             torch.cuda.synchronize()
             quant.launch(q8, qs, x)
             la.launch(q8, k, v, out, tables, lens, workspace=ws, k_scale_cache=ks, v_scale_cache=vs, q_scale_cache=qs)
+            assert L.rvllm_paged_decode_last_form() == 5
             torch.cuda.synchronize()
             outs.append(out)
     finally:

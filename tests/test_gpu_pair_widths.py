@@ -6,9 +6,13 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-# batch tiles of 32 to 160 columns over ragged rows and ragged output channels, one or several tiles per pair, split or not
-@pytest.mark.parametrize("N,K,M", [(512, 512, 129), (512, 512, 1355), (1000, 512, 700), (4096, 512, 2048), (512, 2048, 333),
-                                   (1152, 3456, 500), (2048, 1152, 97), (130, 192, 2000)])
+# (N, K, M, width of the batch tile, pairs that share K): ragged rows and ragged output channels, one or several tiles per pair
+SHAPES = [(512, 512, 129, 32, 1), (512, 512, 1355, 64, 1), (1000, 512, 700, 64, 1), (4096, 512, 2048, 256, 1), (512, 2048, 333, 32, 2),
+          (1152, 3456, 500, 128, 3), (2048, 1152, 97, 32, 1), (130, 192, 2000, 32, 1),
+          (512, 512, 2600, 96, 1), (1152, 1024, 2007, 160, 1)]
+
+
+@pytest.mark.parametrize("N,K,M", [s[:3] for s in SHAPES])
 @pytest.mark.parametrize("residual", [False, True])
 def test_narrow_tiles(N, K, M, residual):
     from rvllm_b200 import gemm
