@@ -155,22 +155,23 @@ int launch_items(const rvattn::Params& p, cudaStream_t s) {
     const long long slots = (long long)p.num_blocks_total * p.block_size;
     const int group = p.heads / p.kv_heads;
     if (!rvua::cache_map(&mk, p.k_cache, slots, p.kv_heads, HD, p.block_size) ||
-        !rvua::cache_map(&mv, p.v_cache, slots, p.kv_heads, HD, p.block_size) ||
-        !rvua::cache_map(&mq, p.q, (long long)p.batch * p.heads, 1, HD, group))  // Q: rows of a KV head's query heads
+        !rvua::cache_map(&mv, p.v_cache, slots, p.kv_heads, HD, p.block_size))
         return rv_fail(RVLLM_E_LAUNCH, "cuTensorMapEncodeTiled failed for the KV cache");
+    if (!rvua::cache_map(&mq, p.q, (long long)p.batch * p.heads, 1, HD, group))  // rows of a KV head's query heads
+        return rv_fail(RVLLM_E_LAUNCH, "cuTensorMapEncodeTiled failed for Q");
     auto kern = rvua::paged_decode_fp8_items_kernel<HD, GT, OutT>;
     using C = rvua::ItemCfg<HD>;
     static RvDeviceOnce smem_once;  // per kernel instantiation and device
     if (rv_allow_smem(smem_once, kern, C::smem_bytes(C::MOST_UNITS)))
         return rv_fail(RVLLM_E_LAUNCH, "cannot raise dynamic shared memory for decode attention");
     const int ring = g_ring_units.load();
-    const long long ctas = (long long)p.kv_heads * p.max_chunks * p.batch;
+    const long long ctas = (long long)p.kv_heads * p.batch;
     int units = ring > 0 ? ring : rvua::pick_units<C>(ctas, rvua::ctas_per_sm<HD, GT>());
     if (units < C::MIN_UNITS) units = C::MIN_UNITS;
     if (units > C::MOST_UNITS) units = C::MOST_UNITS;
     t_last_form = 5;
     const int ordered = p.window_size_left < 0 && p.batch > 1 && p.batch <= rvua::ORDER_MAX;
-    rv_launch(kern, dim3(p.kv_heads, p.max_chunks, p.batch), dim3(rvua::THREADS), (size_t)C::smem_bytes(units), s, dim3(1, 1, 1),
+    rv_launch(kern, dim3(p.kv_heads, 1, p.batch), dim3(rvua::THREADS), (size_t)C::smem_bytes(units), s, dim3(1, 1, 1),
               mk, mv, mq, p, units, ordered);
     return rv_launched("paged_decode_fp8 (tcgen05)");
 }

@@ -1,7 +1,7 @@
 // FP8-KV paged GQA decode attention on tcgen05 / TMEM / TMA: one CTA, many (sequence, KV head) items.
 //
-// The form of paged_decode_fp8_umma.cuh whose chunks do not meet in a cluster: same contract, grid (kv_heads, chunks, batch),
-// chunk rule, tile arithmetic and partial layout.  What differs is how the grid's blocks become work.  A batch of short
+// The form of paged_decode_fp8_umma.cuh for sequences that are not split: same contract, grid (kv_heads, 1, batch), tile arithmetic
+// and partial layout (of one chunk).  What differs is how the grid's blocks become work.  A batch of short
 // contexts is thousands of blocks of one or two tiles, each a chain of dependent latencies (launch, tensor memory,
 // context length -> table -> TMA -> scores -> softmax -> product -> store) of 6-8 us around a microsecond of work.  Here a
 // resident CTA takes over blocks that have not started (clusterlaunchcontrol.try_cancel, the hardware's own queue: no
@@ -30,14 +30,15 @@ constexpr int ITEM_AUX_BYTES = 2048;
 // A value that is the same in all lanes, in a uniform register (where the warp reduction leaves its result)
 __device__ __forceinline__ int uniform(int v) { return (int)__reduce_or_sync(0xffffffffu, (unsigned)v); }
 
-// ---- sequences by falling attended length ------------------------------------------------------------------------------
+// ---- sequences by falling length ---------------------------------------------------------------------------------------
 // Blocks start in grid order, the batch outermost.  Where the grid takes more than one wave, that order is made the order of
 // falling length, so that the longest sequences do not start last (64 sequences of 512 to 32768 tokens, head_dim 256: 1614 us in the
 // callers' order, 1290 in this one).  Nothing is kept: every CTA sorts the batch, by counting, in its first microsecond.
 constexpr int ORDER_MAX = 256;  // sequences it is done for (a thread or two each)
-// Keys that fall with the attended length, then with the sequence's number.  True if this thread saw two lengths.
+// Keys that fall with the length (no window: all of it is attended), then with the sequence's number.  True if this thread saw two lengths.
 __device__ __forceinline__ bool order_keys(const Params& p, int* key, int tid) {
-    const int cap = p.window_size_left >= 0 ? min(p.window_size_left + 1, 0x7fffff) : 0x7fffff, first = min(p.context_lens[0], cap);
+    constexpr int cap = 0x7fffff;
+    const int first = min(p.context_lens[0], cap);
     bool differ = false;
     for (int i = tid; i < ORDER_MAX; i += THREADS) {
         const int len = i < p.batch ? min(p.context_lens[i], cap) : 0;
@@ -60,9 +61,9 @@ __device__ __forceinline__ void order_ranks(const Params& p, const int* key, uin
 }
 
 struct Item {
-    int b, kvh, chunk, nchunks;
+    int b, kvh;
     int t_begin, t_end, tile0, ntiles;  // ntiles 0: nothing attended (fill says what to store), -1: no more items
-    int fill, pad[3];                   // 0: nothing to store, 1: zeros, 2: NaN
+    int fill, pad;                      // 1: zeros, 2: NaN
 };
 
 // Claims a block of the grid that has not started; the 16-byte answer lands at `dst`, counted on `bar`.
@@ -71,7 +72,7 @@ __device__ __forceinline__ void claim_block(void* dst, uint64_t* bar) {
                  "r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ bool claimed_block(const void* src, int& x, int& y, int& z) {
+__device__ __forceinline__ bool claimed_block(const void* src, int& x, int& z) {
     uint32_t ok, bx = 0, by = 0, bz = 0;
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
@@ -84,7 +85,6 @@ __device__ __forceinline__ bool claimed_block(const void* src, int& x, int& y, i
         : "r"(smem_u32(src))
         : "memory");
     x = (int)bx;
-    y = (int)by;
     z = (int)bz;
     return ok != 0;
 }
@@ -176,7 +176,7 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
     uint8_t* claim = aux + 384;                          // 16 bytes: answer of the last claim
     float* red = reinterpret_cast<float*>(aux + 400);    // [2][4][8] tile maxima, then [4][8] sums, [12] masks and flags (108 floats)
     Item* items = reinterpret_cast<Item*>(aux + 832);    // [ITEM_SLOTS]
-    uint8_t* s_perm = aux + 1024;                        // [ORDER_MAX] sequences by falling attended length
+    uint8_t* s_perm = aux + 1024;                        // [ORDER_MAX] sequences by falling length
     int* s_key = reinterpret_cast<int*>(ring);           // [ORDER_MAX] their sort keys, before the ring is used
     static_assert(384 >= (2 * MAX_UNITS + 10 + 2 * ITEM_SLOTS + 1) * 8 + 4 && 400 + 108 * 4 <= 832 &&
                       832 + ITEM_SLOTS * sizeof(Item) <= 1024 && 1024 + ORDER_MAX <= ITEM_AUX_BYTES, "scratch layout");
@@ -244,9 +244,9 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
 
     if (warp == 0) {
         // ------------------------------------------------------------------ scheduler and producer (whole warp)
-        // Lane j owns page j of every tile: one table load and one TMA per lane and panel, issued side by side.
+        // Lane j looks page j of every tile up; one elected lane issues the loads.
         const int ppt = TOK / bs;  // pages per tile (<= 16)
-        int x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
+        int x = blockIdx.x, z = blockIdx.z;
         int slot = 0, use = 0;     // ring position of the next unit
         int n = 0, active = 0, q_sent = 0;  // items published, items with tiles among them, Q loads issued
         uint32_t claims = 0, answers = 0;
@@ -257,27 +257,20 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
             // (one value in all lanes: the loads below are issued by one elected lane from uniform registers)
             Item it;
             x = uniform(x);
-            y = uniform(y);
             it.b = uniform(reorder ? (int)s_perm[z] : z);
             it.kvh = x;
-            it.chunk = y;
-            it.nchunks = 1;
             it.t_begin = it.t_end = it.tile0 = it.ntiles = it.fill = 0;
             if (more) {
                 const int ctx = uniform(p.context_lens[it.b]);
                 if (ctx <= 0 || (p.window_size_left < 0 && (long long)ctx > (long long)bs * p.max_blocks_per_seq)) {
-                    if (y == 0) it.fill = ctx == 0 ? 1 : 2;
+                    it.fill = ctx == 0 ? 1 : 2;
                 } else {
                     int start, len;
                     rvattn::attend_interval(ctx, p.window_size_left, start, len);
-                    it.nchunks = rvattn::chunks_for(len, p.max_chunks, p.min_chunk_tokens);
-                    if (y < it.nchunks) {
-                        const int chunk_size = (len + it.nchunks - 1) / it.nchunks;
-                        it.t_begin = start + y * chunk_size;
-                        it.t_end = min(it.t_begin + chunk_size, start + len);
-                        it.tile0 = (it.t_begin / bs) * bs;  // first tile starts on a page boundary
-                        it.ntiles = it.t_end > it.t_begin ? (it.t_end - it.tile0 + TOK - 1) / TOK : 0;
-                    }
+                    it.t_begin = start;
+                    it.t_end = start + len;
+                    it.tile0 = (it.t_begin / bs) * bs;  // first tile starts on a page boundary
+                    it.ntiles = (it.t_end - it.tile0 + TOK - 1) / TOK;
                 }
             } else {
                 it.ntiles = -1;
@@ -365,7 +358,7 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
             }
             alive = wait_one(claim_bar, (claims - 1) & 1u, 13);
             answers = claims;
-            more = __all_sync(0xffffffffu, alive && claimed_block(claim, x, y, z)) != 0;  // (after a refusal there is no further claim)
+            more = __all_sync(0xffffffffu, alive && claimed_block(claim, x, z)) != 0;  // (after a refusal there is no further claim)
         }
         if (!waited) rv::pdl_wait();
         if (!alive) {  // a wait gave up: this warp's copies in flight land before the block leaves
@@ -584,19 +577,15 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
         while (ntiles >= 0) {
             const int cur = n - 1;  // the record is kept until the item's results are stored
             if (ntiles == 0) {
-                const int fill_code = items[cur & (ITEM_SLOTS - 1)].fill;
-                if (fill_code != 0) {
-                    const float fill = fill_code == 1 ? 0.0f : CUDART_NAN_F;
-                    if (p.force_partial) {
-                        for (int i = tid - 64; i < group * PSTRIDE; i += 128) {
-                            const int hh = i / PSTRIDE, d = i % PSTRIDE;
-                            float* ws = p.workspace + (((size_t)b * p.heads + (size_t)kvh * group + hh) * p.max_chunks) * PSTRIDE;
-                            ws[d] = d < HD ? fill : (d == HD ? -1e20f : 0.0f);
-                        }
-                    } else {
-                        for (int i = tid - 64; i < group * HD; i += 128)
-                            out[((size_t)b * p.heads + (size_t)kvh * group) * HD + i] = rv::T16<OutT>::from_f32(fill);
+                const float fill = items[cur & (ITEM_SLOTS - 1)].fill == 1 ? 0.0f : CUDART_NAN_F;
+                const size_t head0 = (size_t)b * p.heads + (size_t)kvh * group;
+                if (p.force_partial) {
+                    for (int i = tid - 64; i < group * PSTRIDE; i += 128) {
+                        const int d = i % PSTRIDE;
+                        p.workspace[head0 * PSTRIDE + i] = d < HD ? fill : (d == HD ? -1e20f : 0.0f);
                     }
+                } else {
+                    for (int i = tid - 64; i < group * HD; i += 128) out[head0 * HD + i] = rv::T16<OutT>::from_f32(fill);
                 }
                 drop_item(cur);
                 next_item();
@@ -728,7 +717,6 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
             meet();
             const unsigned bad_mask = alive ? (bads[0] | bads[1] | bads[2] | bads[3]) : 0xffffffffu;
             const Item& it = items[cur & (ITEM_SLOTS - 1)];
-            const bool whole = it.nchunks == 1 && !p.force_partial;
             const size_t head0 = (size_t)it.b * p.heads + (size_t)it.kvh * group;
 #pragma unroll
             for (int h = 0; h < HALVES; h++) {
@@ -749,12 +737,12 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
                     if (k < nh) {
                         const float L = sums[k] + sums[8 + k] + sums[16 + k] + sums[24 + k];
                         const bool any_bad = (bad_mask >> k) & 1u;
-                        if (whole) {
+                        if (!p.force_partial) {
                             float v = L > 0.0f ? acc[k] / L : acc[k];
                             if (any_bad) v = CUDART_NAN_F;
                             out[(head0 + k) * HD + d] = rv::T16<OutT>::from_f32(v);
                         } else {
-                            float* ws = p.workspace + ((head0 + k) * p.max_chunks + it.chunk) * PSTRIDE;
+                            float* ws = p.workspace + (head0 + k) * PSTRIDE;
                             ws[d] = any_bad ? CUDART_NAN_F : acc[k];
                             if (d == 0) {
                                 ws[HD] = (m_run[k] - 8.0f) * 0.6931471805599453f;  // back to base e
@@ -794,7 +782,7 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
 // 12-layer stack: 1465 / 1476 us per step).
 template <int HD, int GT> inline bool prefer_items(const Params& p) {
     if (p.max_chunks > 1 || p.amax_out) return false;
-    const long long ctas = (long long)p.kv_heads * p.max_chunks * p.batch;
+    const long long ctas = (long long)p.kv_heads * p.batch;
     const int fit = (228 * 1024) / (Cfg<HD>::smem_bytes(pick_units<Cfg<HD>>(ctas, ctas_per_sm<HD, GT>())) + 1024);
     const long long resident = (long long)(fit < ctas_per_sm<HD, GT>() ? fit : ctas_per_sm<HD, GT>()) * rv::SMS;
     return ctas > (p.window_size_left < 0 ? resident : 2 * resident);

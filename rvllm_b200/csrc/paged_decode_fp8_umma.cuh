@@ -7,7 +7,7 @@
 // does not bring enough warps to hide that.  Here a CTA moves and multiplies whole pages:
 //
 //   tile    = 128 tokens of one KV head (whole cache pages, first and last tile masked).
-//   warp 0  : producer.  One lane looks the pages up in the block table and issues one TMA
+//   warp 0  : producer.  Lane j looks page j of a tile up in the block table, one elected lane issues a TMA
 //             (cp.async.bulk.tensor.3d, 128-byte swizzle) per page and 128-byte panel of K and of V
 //             into a ring of 16 KB units; completion is counted on an mbarrier per unit.
 //   warp 1  : MMA issuer.  scores^T[128 tokens x 16 head columns] = K_tile . Q^T with
@@ -379,9 +379,8 @@ paged_decode_fp8_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer (whole warp)
-        // Lane j owns page j of every tile: one table load and one TMA per lane and panel, issued side
-        // by side, instead of one thread walking the pages (serial address arithmetic and TMA issue
-        // cost ~2 us per tile that way, more than the loads themselves).
+        // Lane j looks page j of every tile up, all of a tile's table entries side by side; one elected lane issues the loads
+        // (load_pages above).
         if (ntiles > 0) {
             const int ppt = TOK / bs;  // pages per tile (<= 16)
             const bool one = rv::elect_one();
