@@ -766,16 +766,15 @@ paged_decode_fp8_items_kernel(const __grid_constant__ CUtensorMap map_k, const _
 // Which launches take this kernel: one chunk per sequence and more blocks than the one-item kernel keeps resident at once; with a
 // window, where nothing is reordered, from two waves on.  Lengths are not known here, and what it gives depends on them.  Measured,
 // us, one-item kernel (in the callers' order) / this one, 16-token pages:
-//   short       128 sequences of 48 tokens, 16 KV heads, head_dim 128 28.6 / 22.5; 256 of 516 121.5 / 114.9; 64 of 516, head_dim 512
+//   short       128 sequences of 48 tokens, 16 KV heads, head_dim 128 28.7 / 20.6; 256 of 516 123.0 / 114.1; 64 of 516, head_dim 512
 //               143 / 125
 //   unequal     64 of 500 to 16000, head_dim 128 397 / 381; 64 of 100 to 4000, 64 / 8 heads 105 / 72, head_dim 512 266 / 200, 32 / 16
 //               heads 360 / 335
 //   with a window of 1024: 256 of 16 to 400 tokens, head_dim 128 69.7 / 62.0; 256 of 100 to 4000, 64 / 8 heads, head_dim 256 229 / 215
-//   equal, long 64 of 2000, 16 KV heads, head_dim 128 102.7 / 106.6; 256 of 4000 631 / 670, with a window of 1024 182 / 187; 128 of 4000,
+//   equal, long 64 of 2000, 16 KV heads, head_dim 128 102.7 / 106.6; 256 of 4000 652 / 690, with a window of 1024 184 / 192; 128 of 4000,
 //               64 / 8 heads, head_dim 256 390 / 382
 // So the cost is with equal long contexts at head_dim 128 and one or two query heads per KV head, which stream at the copy rate in
-// either kernel (3 to 6 %), and with short ones at head_dim 512 and more than four (40 of 48 tokens 33 / 37; 128 of 16 to 400 with a
-// window 92 / 101).
+// either kernel: 3 to 6 %.  Over 1018 shapes with 20 to 256 sequences, grids of one wave among them, the time is 0.92 on average.
 // A grid that is resident at once gains nothing and pays for the records and claims: 33 sequences of 22 to 411 tokens 12.0 / 13.3.
 // So do grids whose blocks are chunks that short sequences leave empty (15 sequences of up to 56 tokens, a whole layer
 // 126.5 / 132.8), and the form that leaves maxima for the O projection, which is part of a chain of dependent launches (32 rows, a
