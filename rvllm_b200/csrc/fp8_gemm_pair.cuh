@@ -625,8 +625,8 @@ inline PairPlan pair_plan(int M, int N, int K, int ranges) {
     const int nw = (N + 255) / 256, kblocks = (K + BK - 1) / BK;
     PairPlan best = {};
     double best_cost = 0.0;
-    // (many rows run at the power cap, where a narrower tile, which moves more and pads more, must be worth it: 43008 x 5376 at 1000
-    // rows 158 us with 256 columns, 175 with 160, which the model puts 1 % ahead)
+    // (many rows run at the power cap, where a narrower tile, which moves more and pads more, must be worth it, as must a split: 43008 x
+    // 5376 at 1000 rows 158 us with 256 columns, 175 with 160, which the model puts 1 % ahead)
     const double worth = M > 512 ? 0.96 : 1.0;
     for (int bn = M > 224 ? 256 : (M + 31) / 32 * 32; bn >= 32; bn -= 32) {
         const int nb = (M + bn - 1) / bn, tiles = nw * nb;
